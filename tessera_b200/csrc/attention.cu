@@ -18,6 +18,7 @@
 // them with its own chunk count and buffers (src/core/decode_internal.hpp:299-374).
 #include <cuda_fp16.h>
 
+#include "attention.cuh"
 #include "codec.cuh"
 #include "launch.h"
 #include "tessera_b200.h"
@@ -25,16 +26,9 @@
 namespace tsr {
 namespace {
 
-constexpr int kAttnWarps = 8, kAttnMaxGroup = 8;  // heads / kv_heads <= 8
+constexpr int kAttnWarps = 8;
 constexpr int kAttnMaxSplits = 64, kAttnMinKeys = 64;  // chunks the whole-attention entry cuts the key range into
-constexpr float kNullMax = -1e30f;  // running max before the first key, as the reference's kernels have it
 
-enum : int { kKvF32 = 0, kKvF16 = 1, kKvFp8 = 2, kKvInt8 = 3, kKvInt4 = 4 };
-
-template <int KV>
-__host__ __device__ constexpr int kv_bits() {
-  return KV == kKvF32 ? 32 : KV == kKvF16 ? 16 : KV == kKvInt4 ? 4 : 8;
-}
 __host__ __device__ constexpr int cmin(int a, int b) { return a < b ? a : b; }
 
 // BYTES (2, 4, 8 or 16) of a cache row into words; the address is a multiple of BYTES.
@@ -80,25 +74,6 @@ __device__ __forceinline__ void decode(const uint32_t (&w)[4], float (&out)[N]) 
     }
   }
 }
-
-struct AttnParams {
-  const float* q;
-  const void* k;
-  const void* v;
-  const float* ks;
-  const float* vs;
-  // partial of (query row i, head h, chunk s) at base = (i * heads + h) * splits + s: pacc[base * head_dim ..],
-  // pmax[base], psum[base]; an empty chunk is the null partial (0, kNullMax, 0)
-  // (the layout of the reference's split kernels, src/backends/rocm/rocm_kernels_basic.cpp:278-330)
-  float* pacc;
-  float* pmax;
-  float* psum;
-  int m, n, heads, kv_heads, head_dim, window, causal, splits;
-  unsigned long long q_base, row_base;
-};
-
-constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
-constexpr float kNoKey = -3.0e38f;  // score of a key outside the chunk, and the running max before the first key
 
 // One CTA: one query row, one kv head (all G query heads of its group), one chunk of the key range.
 // Scores: 8 lanes share a key (each 1/8 of head_dim in 16-byte pieces, a row read as contiguous 128-byte
@@ -429,15 +404,17 @@ int run_attention(int kvkind, const float* q, const void* k, const void* v, cons
                   const float* gate, uint64_t m, uint64_t n, uint64_t heads, uint64_t kv_heads, uint64_t head_dim,
                   uint64_t q_base, uint64_t row_base, uint64_t window, uint64_t causal, cudaStream_t st) {
   if (!out) return kInvalidArgument;
+  AttnParams p;
+  if (int rc = check_attention(kvkind, q, k, v, ks, vs, m, n, heads, kv_heads, head_dim, q_base, row_base, window, causal, 1, &p))
+    return rc;
+  const int tile = attention_tile(kvkind, p, out, gate, st);
+  if (tile != kUnsupportedFeature) return tile;
   // as many chunks as keep a CTA busy with kAttnMinKeys keys, counted on the longest row's range
   const uint64_t span = window != 0 && window < n ? window : n;
   uint64_t splits = span / kAttnMinKeys;
   if (splits < 1) splits = 1;
   if (splits > kAttnMaxSplits) splits = kAttnMaxSplits;
-  AttnParams p;
-  if (int rc = check_attention(kvkind, q, k, v, ks, vs, m, n, heads, kv_heads, head_dim, q_base, row_base, window, causal,
-                               splits, &p))
-    return rc;
+  p.splits = static_cast<int>(splits);
   const size_t parts = m * heads * splits;
   const size_t acc_bytes = parts * head_dim * 4, stat_bytes = (parts * 4 + 255) / 256 * 256;
   unsigned char* scratch = stream_scratch(st, acc_bytes + 2 * stat_bytes, 2);

@@ -218,3 +218,50 @@ def test_written_cache_feeds_attention(backend, oracle):
     (kc, ks), (vc, vs) = oracle.quantize_rows(0, kf), oracle.quantize_rows(0, vf)
     want = oracle.attention(2, q, kc, vc, 1, n, heads, kv_heads, head_dim, n - 1, 0, True, ks, vs)
     assert near(backend.download(out, np.float32, heads * head_dim).reshape(1, -1), want)
+
+
+# (m, n, heads, kv_heads, head_dim, q_base, window): the fewest rows the tile takes, a second row tile of four rows, one
+# head per kv head on a first chunk, a window that starts inside tiles, query rows past the cache, eight heads per kv
+# head over many chunks
+BATCHES = [(4, 2100, 24, 4, 256, 2096, 0), (22, 400, 24, 4, 256, 378, 0), (130, 130, 8, 8, 128, 0, 0), (101, 1500, 16, 2, 128, 1399, 300),
+           (57, 160, 24, 4, 256, 120, 0), (129, 700, 4, 4, 128, 500, 130), (16, 2049, 16, 2, 256, 2033, 0)]
+
+
+@pytest.mark.parametrize("fmt", [1, 2, 3, 4])
+@pytest.mark.parametrize("m,n,heads,kv_heads,head_dim,q_base,window", BATCHES)
+def test_batches_on_the_tensor_pipe(backend, oracle, fmt, m, n, heads, kv_heads, head_dim, q_base, window):
+    """Batches of query rows (two binary16 terms per query element and weight, exact cache elements): fp32 rounding."""
+    g = np.random.default_rng(50 + fmt + m)
+    q = g.standard_normal((m, heads * head_dim)).astype(np.float32) * np.float32(10.0) ** g.integers(-3, 2, (m, 1)).astype(np.float32)
+    k, v, ks, vs = make_cache(g, fmt, n, kv_heads * head_dim)
+    y = device_attention(backend, fmt, q, k, v, ks, vs, m, n, heads, kv_heads, head_dim, q_base, window, True, row_base=1)
+    r = oracle.attention(fmt, q, k, v, m, n, heads, kv_heads, head_dim, q_base, window, True, ks, vs)
+    assert near(y, r)
+
+
+def test_batch_without_causal_mask(backend, oracle):
+    g = np.random.default_rng(60)
+    m, n, heads, kv_heads, head_dim = 320, 333, 8, 2, 128
+    q = g.standard_normal((m, heads * head_dim)).astype(np.float32)
+    k, v, ks, vs = make_cache(g, 1, n, kv_heads * head_dim)
+    y = device_attention(backend, 1, q, k, v, ks, vs, m, n, heads, kv_heads, head_dim, 0, 0, False)
+    assert near(y, oracle.attention(1, q, k, v, m, n, heads, kv_heads, head_dim, 0, 0, False, ks, vs))
+
+
+@pytest.mark.parametrize("fmt", [1, 4])
+def test_nonfinite_values_reach_only_the_rows_that_see_them(backend, oracle, fmt):
+    """A NaN value in key 250 and an infinite fp16 key 255: rows at positions below see neither."""
+    g = np.random.default_rng(70 + fmt)
+    m, n, heads, kv_heads, head_dim = 120, 300, 8, 2, 128
+    q = np.abs(g.standard_normal((m, heads * head_dim))).astype(np.float32)
+    k, v, ks, vs = make_cache(g, fmt, n, kv_heads * head_dim)
+    if fmt == 1:
+        v.view(np.float16)[250] = np.nan
+        k.view(np.float16)[255, 3] = -np.inf
+    else:
+        v[250] = 0x7F
+    y = device_attention(backend, fmt, q, k, v, ks, vs, m, n, heads, kv_heads, head_dim, n - m, 0, True)
+    r = oracle.attention(fmt, q, k, v, m, n, heads, kv_heads, head_dim, n - m, 0, True, ks, vs).reshape(y.shape)
+    clean = 250 - (n - m)
+    assert near(y[:clean], r[:clean])
+    assert np.isnan(y[clean:]).all() and np.isnan(r[clean:]).all()
