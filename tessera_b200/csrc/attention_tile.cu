@@ -580,6 +580,10 @@ int launch_tile_d(const AttnTileParams& tp, cudaStream_t st) {
   return tp.a.head_dim == 256 ? launch_tile<KV, 256>(tp, st) : launch_tile<KV, 128>(tp, st);
 }
 
+bool overlap(const void* a, size_t an, const void* b, size_t bn) {
+  const auto *x = static_cast<const unsigned char*>(a), *y = static_cast<const unsigned char*>(b);
+  return x < y + bn && y < x + an;
+}
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 }  // namespace
@@ -598,6 +602,18 @@ int attention_tile(int kvkind, AttnParams p, float* out, const float* gate, cuda
   // 16-byte pieces of q, the cache and the output; the chunk kernel takes what is not aligned.
   if (kvkind == kKvF32 || p.m < 4 || static_cast<double>(p.m) * span * p.kv_heads * p.head_dim < 8.0e6 || !aligned16(p.q) ||
       !aligned16(p.k) || !aligned16(p.v) || !aligned16(out))
+    return kUnsupportedFeature;
+  // With one chunk the result is written while other CTAs still read their queries and the cache.  In place over q is
+  // fine (a CTA reads its own rows before it writes them); any other overlap stays with the chunk kernel, whose merge
+  // starts when everything has been read.
+  const size_t out_bytes = static_cast<size_t>(p.m) * p.heads * p.head_dim * 4;
+  const size_t cache_bytes = static_cast<size_t>(p.n) * p.kv_heads * p.head_dim * (kvkind == kKvF16 ? 4 : kvkind == kKvInt4 ? 1 : 2) / 2;
+  const float *rows_q = p.q + p.row_base * p.heads * p.head_dim, *rows_out = out + p.row_base * p.heads * p.head_dim;
+  const size_t scale_bytes = kvkind == kKvF16 ? 0 : static_cast<size_t>(p.n) * 4;
+  if ((rows_out != rows_q && overlap(rows_out, out_bytes, rows_q, out_bytes)) || overlap(rows_out, out_bytes, p.k, cache_bytes) ||
+      overlap(rows_out, out_bytes, p.v, cache_bytes) ||
+      (scale_bytes != 0 && (overlap(rows_out, out_bytes, p.ks, scale_bytes) || overlap(rows_out, out_bytes, p.vs, scale_bytes))) ||
+      (gate != nullptr && overlap(rows_out, out_bytes, gate + p.row_base * p.heads * p.head_dim, out_bytes)))
     return kUnsupportedFeature;
   static const int sms = [] {
     int dev = 0, v = 0;

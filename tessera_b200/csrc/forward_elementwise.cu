@@ -65,6 +65,58 @@ rmsnorm_gated_kernel(const float* __restrict__ x, const float* __restrict__ w, c
   }
 }
 
+// Head-sized rows (P x 32 columns, P = 4 or 8) with a warp per row: lane c holds columns c, c + 32, ...  The squares are
+// added in block_sum's order -- each run of 32 by a butterfly, the runs by the butterfly of its first warp -- so the
+// results are the ones of the CTA-per-row kernels bit for bit.  A CTA of 256 threads per row of 128 left half of its
+// threads idle and paid two barriers a row: 8192 rows of 128 took 11.0 us (l2norm) and 24576 took 37.0 us
+// (rmsnorm_gated); here 4.2 and 10.0 us, the latter 38 MB at 3.8 TB/s.
+template <int P>
+__device__ __forceinline__ float head_square_sum(const float (&x)[P]) {
+  float s[P];
+#pragma unroll
+  for (int i = 0; i < P; ++i) s[i] = fmaf(x[i], x[i], 0.0f);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int i = 0; i < P; ++i) s[i] += __shfl_xor_sync(0xFFFFFFFFu, s[i], o);
+  if constexpr (P == 8)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) s[i] += s[i + 4];
+  return (s[0] + s[2]) + (s[1] + s[3]);
+}
+constexpr int kHeadRows = 8;  // rows (warps) per CTA
+template <int P>
+__global__ void __launch_bounds__(kHeadRows * 32)
+l2norm_heads_kernel(const float* __restrict__ x, float* __restrict__ y, unsigned rows, float eps, float scale) {
+  const unsigned r = blockIdx.x * kHeadRows + (threadIdx.x >> 5);
+  if (r >= rows) return;
+  const size_t base = static_cast<size_t>(r) * (P * 32) + (threadIdx.x & 31);
+  float v[P];
+#pragma unroll
+  for (int i = 0; i < P; ++i) v[i] = x[base + i * 32];
+  const float gain = scale / sqrtf(head_square_sum<P>(v) + eps);
+#pragma unroll
+  for (int i = 0; i < P; ++i) y[base + i * 32] = v[i] * gain;
+}
+template <int P>
+__global__ void __launch_bounds__(kHeadRows * 32)
+rmsnorm_gated_heads_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ gate,
+                           float* __restrict__ y, unsigned rows, float eps, size_t gbase, size_t ybase) {
+  const unsigned r = blockIdx.x * kHeadRows + (threadIdx.x >> 5);
+  if (r >= rows) return;
+  const int lane = threadIdx.x & 31;
+  const size_t base = static_cast<size_t>(r) * (P * 32) + lane;
+  float v[P], g[P];
+#pragma unroll
+  for (int i = 0; i < P; ++i) v[i] = x[base + i * 32], g[i] = gate[gbase + base + i * 32];
+  const float gain = 1.0f / sqrtf(head_square_sum<P>(v) / static_cast<float>(P * 32) + eps);
+#pragma unroll
+  for (int i = 0; i < P; ++i) {
+    const float silu = g[i] / (1.0f + expf(-g[i]));
+    y[ybase + base + i * 32] = v[i] * gain * w[lane + i * 32] * silu;
+  }
+}
+
 // alpha = exp(a_log[h] * softplus(alpha_raw + dt[h])), beta = sigmoid(beta_raw) (SsmGateRef)
 __global__ void ssm_gate_kernel(const float* __restrict__ a_log, const float* __restrict__ dt,
                                 const float* __restrict__ alpha_raw, const float* __restrict__ beta_raw,
@@ -97,6 +149,17 @@ __global__ void repeat_heads_kernel(const float* __restrict__ in, float* __restr
   const size_t e = i % head_k_dim, rh = i / head_k_dim;
   const size_t h = rh % num_v_heads, r = rh / num_v_heads;
   out[i] = in[(r * num_k_heads + h % num_k_heads) * head_k_dim + e];
+}
+
+// The same, four elements a thread with 32-bit index arithmetic (head_k_dim a multiple of 4, 16-byte aligned buffers,
+// fewer than 2^31 elements): 512 rows of 48 heads of 128 in 5.6 us against 17.0.
+__global__ void __launch_bounds__(256)
+repeat_heads4_kernel(const float4* __restrict__ in, float4* __restrict__ out, unsigned num_v_heads, unsigned dim4,
+                     unsigned num_k_heads, unsigned total4) {
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= total4) return;
+  const unsigned rh = i / dim4, e = i - rh * dim4, r = rh / num_v_heads, h = rh - r * num_v_heads;
+  out[i] = in[(r * num_k_heads + h % num_k_heads) * dim4 + e];
 }
 
 // Out[row] = table[ids[row]] as fp32, a zero row for an id outside the table
@@ -289,6 +352,196 @@ delta_step_heads_kernel(float* __restrict__ s, const float* __restrict__ k, cons
   }
 }
 
+// The same steps with dk = 128.  The steps are a serial chain, so what counts is a step's latency and its instructions:
+// the kernel above meets in shared memory twice a step behind five barriers and took 2.2 us a row (512 rows of 48 heads
+// 1135 us; here 155 us).  Sixteen lanes share two state columns, eight rows of each as four
+// register pairs for the two-wide fp32 multiply-add (fma.rn.f32x2), so a step's sums over dk are register sums and a few
+// shuffles and no warp waits for another; the vectors of kDeltaSteps steps arrive by cp.async one block ahead.  With
+// c = beta (v - alpha r):  S' = alpha S + k c^T, o = S'^T q; alpha S and the products with q are off the chain.
+// Measured lay-outs (512 rows): one column over eight lanes 195 us (k and q cost 1 KB of shared memory a column and
+// step), two columns over 4 / 8 / 16 lanes 172 / 165 / 155 us (fewer, longer warps leave the chain exposed).
+constexpr int kDeltaSteps = 16, kDeltaRowCols = 16, kDeltaDk = 128;
+constexpr int kDeltaLanes = 16;  // lanes that share a pair of columns
+constexpr int kDeltaRowThreads = kDeltaRowCols / 2 * kDeltaLanes;
+constexpr int kDeltaPairs = kDeltaDk / kDeltaLanes / 2;  // register pairs of a column in a lane
+constexpr int kDeltaSpan = kDeltaLanes * 4;              // rows between a lane's float4s
+struct DeltaBlock {
+  float k[kDeltaSteps][kDeltaDk], q[kDeltaSteps][kDeltaDk], v[kDeltaSteps][kDeltaRowCols], alpha[kDeltaSteps], beta[kDeltaSteps];
+};
+__device__ __forceinline__ unsigned long long f32x2_fma(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ unsigned long long f32x2_mul(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ unsigned long long f32x2_add(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ unsigned long long f32x2_pack(float x, float y) {
+  unsigned long long d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
+  return d;
+}
+__device__ __forceinline__ float f32x2_sum(unsigned long long a) {
+  float x, y;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
+  return x + y;
+}
+__device__ __forceinline__ void copy_async(void* dst, const float* src, bool wide) {
+  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+  if (wide) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
+}
+
+__global__ void __launch_bounds__(kDeltaRowThreads)
+delta_step_rows_kernel(float* __restrict__ s, const float* __restrict__ k, const float* __restrict__ v,
+                       const float* __restrict__ q, float* __restrict__ o, const float* __restrict__ alpha,
+                       const float* __restrict__ beta, int heads, int dv, int rows, size_t sbase, size_t sstride,
+                       size_t abase) {
+  __shared__ __align__(16) DeltaBlock block[2];
+  const int slabs = dv / kDeltaRowCols, h = blockIdx.x / slabs, col0 = (blockIdx.x % slabs) * kDeltaRowCols;
+  // columns d and d + 1, rows kDeltaSpan i + 4 sub + {0..3}
+  const int tid = threadIdx.x, sub = tid % kDeltaLanes, col = tid / kDeltaLanes * 2, d = col0 + col;
+  const bool odd = (sub & 1) != 0;  // the column whose sums end in this lane
+  auto stage = [&](int t0, DeltaBlock& b) {
+    const int steps = min(kDeltaSteps, rows - t0);
+    constexpr int kVec = kDeltaDk / 4, kVVec = kDeltaRowCols / 4;
+    for (int x = tid; x < steps * kVec; x += kDeltaRowThreads) {
+      const int t = x / kVec, c = (x % kVec) * 4;
+      const size_t at = (static_cast<size_t>(t0 + t) * heads + h) * kDeltaDk + c;
+      copy_async(&b.k[t][c], k + at, true);
+      copy_async(&b.q[t][c], q + at, true);
+    }
+    for (int x = tid; x < steps * kVVec; x += kDeltaRowThreads) {
+      const int t = x / kVVec, c = (x % kVVec) * 4;
+      copy_async(&b.v[t][c], v + (static_cast<size_t>(t0 + t) * heads + h) * dv + col0 + c, true);
+    }
+    if (tid < kDeltaSteps) {
+      if (tid < steps) copy_async(&b.alpha[tid], alpha + abase + static_cast<size_t>(t0 + tid) * heads + h, false);
+    } else if (tid - kDeltaSteps < steps) {
+      copy_async(&b.beta[tid - kDeltaSteps], beta + abase + static_cast<size_t>(t0 + tid - kDeltaSteps) * heads + h, false);
+    }
+  };
+  stage(0, block[0]);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  const size_t state = sbase + static_cast<size_t>(h) * kDeltaDk * dv + d;
+  unsigned long long st[2][kDeltaPairs];  // [column][rows kDeltaSpan (i / 2) + 4 sub + 2 (i % 2) + {0, 1}]
+#pragma unroll
+  for (int i = 0; i < kDeltaPairs; ++i) {
+    const float* src = s + state + static_cast<size_t>(kDeltaSpan * (i >> 1) + 4 * sub + 2 * (i & 1)) * dv;
+    st[0][i] = f32x2_pack(src[0], src[dv]);
+    st[1][i] = f32x2_pack(src[1], src[dv + 1]);
+  }
+  auto store_state = [&](float* dst) {
+#pragma unroll
+    for (int i = 0; i < kDeltaPairs; ++i) {
+      float* at = dst + static_cast<size_t>(kDeltaSpan * (i >> 1) + 4 * sub + 2 * (i & 1)) * dv;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        float x, y;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(st[c][i]));
+        at[c] = x;
+        at[dv + c] = y;
+      }
+    }
+  };
+  // Pairs of sums over their lanes, one for each column: the first column's ends in the even lanes, the second's in
+  // the odd.  A step's output is reduced together with the next step's r: shuffles issue in order, and on their own the
+  // three of the output sat between two steps of the chain.
+  float out_part[2] = {0.0f, 0.0f};  // of the step before
+  auto reduce = [&](float& x, float& y, const float (&xs)[2], const float (&ys)[2]) {
+    const float xo = __shfl_xor_sync(0xFFFFFFFFu, odd ? xs[0] : xs[1], 1), yo = __shfl_xor_sync(0xFFFFFFFFu, odd ? ys[0] : ys[1], 1);
+    x = (odd ? xs[1] : xs[0]) + xo, y = (odd ? ys[1] : ys[0]) + yo;
+#pragma unroll
+    for (int l = 2; l < kDeltaLanes; l <<= 1) {
+      const float x2 = __shfl_xor_sync(0xFFFFFFFFu, x, l), y2 = __shfl_xor_sync(0xFFFFFFFFu, y, l);
+      x += x2, y += y2;
+    }
+  };
+  float* o_at = o + static_cast<size_t>(h) * dv + d + sub;  // of the step before
+  const size_t o_step = static_cast<size_t>(heads) * dv;
+  o_at -= o_step;
+  for (int t0 = 0, n = 0; t0 < rows; t0 += kDeltaSteps, ++n) {
+    if (t0 + kDeltaSteps < rows) stage(t0 + kDeltaSteps, block[(n + 1) & 1]);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();  // this block has arrived for everybody
+    const DeltaBlock& b = block[n & 1];
+    const int steps = min(kDeltaSteps, rows - t0);
+    auto load = [&](unsigned long long (&x)[kDeltaPairs], const float* row) {
+#pragma unroll
+      for (int i = 0; i < kDeltaPairs / 2; ++i) {
+        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(row + kDeltaSpan * i + 4 * sub);
+        x[2 * i] = w.x, x[2 * i + 1] = w.y;
+      }
+    };
+    unsigned long long k_next[kDeltaPairs];
+    load(k_next, b.k[0]);
+    float a_next = b.alpha[0], be_next = b.beta[0], v_next = b.v[0][col + (odd ? 1 : 0)];
+#pragma unroll 2
+    for (int t = 0; t < steps; ++t) {
+      unsigned long long kk[kDeltaPairs], qq[kDeltaPairs];
+#pragma unroll
+      for (int i = 0; i < kDeltaPairs; ++i) kk[i] = k_next[i];
+      const float a = a_next, be = be_next, vb = v_next;
+      const int tn = min(t + 1, kDeltaSteps - 1);  // (a block's last step loads something it does not use)
+      load(qq, b.q[t]);
+      load(k_next, b.k[tn]);
+      a_next = b.alpha[tn], be_next = b.beta[tn], v_next = b.v[tn][col + (odd ? 1 : 0)];
+      float part[2];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        unsigned long long r[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) r[i] = f32x2_mul(st[c][i], kk[i]);
+#pragma unroll
+        for (int i = 4; i < kDeltaPairs; ++i) r[i & 3] = f32x2_fma(st[c][i], kk[i], r[i & 3]);
+        part[c] = f32x2_sum(f32x2_add(f32x2_add(r[0], r[1]), f32x2_add(r[2], r[3])));
+      }
+      const unsigned long long aa = f32x2_pack(a, a);
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int i = 0; i < kDeltaPairs; ++i) st[c][i] = f32x2_mul(st[c][i], aa);
+      float read, out;
+      reduce(read, out, part, out_part);
+      const float mine = be * (vb - a * read);
+      const float other = __shfl_xor_sync(0xFFFFFFFFu, mine, 1);
+      if (sub < 2 && t0 + t > 0) *o_at = out;
+      o_at += o_step;
+      const float c0 = odd ? other : mine, c1 = odd ? mine : other;
+      const unsigned long long cc[2] = {f32x2_pack(c0, c0), f32x2_pack(c1, c1)};
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        unsigned long long o0 = 0ull, o1 = 0ull;
+#pragma unroll
+        for (int i = 0; i < kDeltaPairs; i += 2) {
+          st[c][i] = f32x2_fma(kk[i], cc[c], st[c][i]);
+          st[c][i + 1] = f32x2_fma(kk[i + 1], cc[c], st[c][i + 1]);
+          o0 = f32x2_fma(st[c][i], qq[i], o0);
+          o1 = f32x2_fma(st[c][i + 1], qq[i + 1], o1);
+        }
+        out_part[c] = f32x2_sum(f32x2_add(o0, o1));
+      }
+      if (sstride != 0) store_state(s + state + (static_cast<size_t>(t0 + t) + 1) * sstride);
+    }
+    __syncthreads();  // everybody is done with the block before it is filled again
+  }
+  {
+    const float none[2] = {0.0f, 0.0f};
+    float read, out;
+    reduce(read, out, none, out_part);
+    if (sub < 2) *o_at = out;
+  }
+  if (sstride == 0) store_state(s + state);
+}
+
 // conv1d_state: current-step causal depthwise convolution with the history kept on the device, SiLU and
 // the q / k / v split; `rows` steps advance the history in turn.  One thread per channel; W in checkpoint
 // tap order (tap 0 oldest), history newest first, (width - 1) samples per channel; with hist_stride != 0
@@ -318,6 +571,65 @@ __global__ void conv1d_state_kernel(const float* __restrict__ qkv, const float* 
       for (size_t i = 0; i < stride; ++i) hist_hist[(t + 1) * hist_stride + hbase + i] = hist[hbase + i];
   }
 }
+
+// conv1d_state with W taps known at compile time: a thread walks over kConvRows rows of a channel with the last W - 1
+// samples in registers, so rows run in parallel (the kernel above takes a channel's rows in turn and moves the history
+// through memory: 512 rows of 10240 channels took 613 us on 40 CTAs, here 14 us, 42 MB at 3.0 TB/s).  The first chunk's
+// threads read the old history and write the new one, which for rows >= W - 1 is made of input rows alone.
+constexpr int kConvRows = 16;
+template <int W>
+__global__ void __launch_bounds__(256)
+conv1d_rows_kernel(const float* __restrict__ qkv, const float* __restrict__ w, float* __restrict__ hist, float* __restrict__ q,
+                   float* __restrict__ k, float* __restrict__ v, float* __restrict__ hist_hist, size_t conv_dim,
+                   size_t key_dim, size_t qkv_offset, size_t rows, size_t hist_stride) {
+  const size_t c = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (c >= conv_dim) return;
+  const size_t t0 = static_cast<size_t>(blockIdx.y) * kConvRows, value_dim = conv_dim - 2 * key_dim;
+  const float* src = qkv + qkv_offset + c;
+  float tap[W], past[W - 1], old[W - 1];  // past[i]: the sample i + 1 rows ago
+#pragma unroll
+  for (int i = 0; i < W; ++i) tap[i] = w[c * W + i];
+#pragma unroll
+  for (int i = 0; i < W - 1; ++i) {
+    old[i] = t0 < W - 1 ? hist[c * (W - 1) + i] : 0.0f;
+    past[i] = t0 >= static_cast<size_t>(i) + 1 ? src[(t0 - i - 1) * conv_dim] : 0.0f;
+  }
+  if (t0 == 0) {
+#pragma unroll
+    for (int i = 0; i < W - 1; ++i) past[i] = old[i];
+  }
+  float* dst;
+  size_t pitch;
+  if (c < key_dim) dst = q + c, pitch = key_dim;
+  else if (c < 2 * key_dim) dst = k + (c - key_dim), pitch = key_dim;
+  else dst = v + (c - 2 * key_dim), pitch = value_dim;
+  float now[kConvRows];
+#pragma unroll
+  for (int i = 0; i < kConvRows; ++i) now[i] = t0 + i < rows ? src[(t0 + i) * conv_dim] : 0.0f;
+#pragma unroll
+  for (int i = 0; i < kConvRows; ++i) {
+    const size_t t = t0 + i;
+    if (t < rows) {
+      float acc = __fmul_rn(tap[W - 1], now[i]);
+#pragma unroll
+      for (int j = 1; j < W; ++j) acc = fmaf(tap[W - 1 - j], past[j - 1], acc);
+      dst[t * pitch] = acc / (1.0f + expf(-acc));
+#pragma unroll
+      for (int j = W - 2; j > 0; --j) past[j] = past[j - 1];
+      past[0] = now[i];
+      if (hist_stride != 0) {
+#pragma unroll
+        for (int j = 0; j < W - 1; ++j) hist_hist[(t + 1) * hist_stride + c * (W - 1) + j] = past[j];
+      }
+    }
+  }
+  if (t0 == 0) {
+#pragma unroll
+    for (int i = 0; i < W - 1; ++i)  // `past` of this chunk where it is the only one, else the last input rows
+      hist[c * (W - 1) + i] = rows <= kConvRows ? past[i] : src[(rows - 1 - i) * conv_dim];
+  }
+}
+static_assert(kConvRows >= 3, "the chunks after the first start beyond the history");
 
 // The steps between a linear-attention layer's input projections and its state step in one launch: CTA b takes
 // channels [b cols, (b + 1) cols) of the convolution (cols = the heads' width = blockDim): the first k_heads CTAs
@@ -452,6 +764,7 @@ top_k_rows_kernel(const float* __restrict__ logits, uint32_t* __restrict__ ids, 
 
 unsigned blocks_of(size_t n) { return static_cast<unsigned>((n + 255) / 256); }
 bool fits31(uint64_t v) { return v > 0 && v <= 0x7FFFFFFFull; }
+bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 }  // namespace
 
@@ -481,16 +794,22 @@ int tsr_sigmoid_gate(const float* a, const float* g, float* o, uint64_t n, void*
 
 int tsr_l2norm(const float* x, float* y, uint64_t rows, uint64_t cols, float eps, float scale, void* stream) {
   if (!x || !y || !fits31(rows) || !fits31(cols) || !(eps >= 0.0f)) return kInvalidArgument;
-  l2norm_kernel<<<static_cast<unsigned>(rows), 256, 0, static_cast<cudaStream_t>(stream)>>>(x, y, static_cast<int>(cols),
-                                                                                            eps, scale);
+  auto st = static_cast<cudaStream_t>(stream);
+  const unsigned n = static_cast<unsigned>(rows), ctas = (n + kHeadRows - 1) / kHeadRows;
+  if (cols == 128) l2norm_heads_kernel<4><<<ctas, kHeadRows * 32, 0, st>>>(x, y, n, eps, scale);
+  else if (cols == 256) l2norm_heads_kernel<8><<<ctas, kHeadRows * 32, 0, st>>>(x, y, n, eps, scale);
+  else l2norm_kernel<<<n, 256, 0, st>>>(x, y, static_cast<int>(cols), eps, scale);
   return check_launch();
 }
 
 int tsr_rmsnorm_gated(const float* x, const float* w, const float* gate, float* y, uint64_t rows, uint64_t cols,
                       float eps, uint64_t gbase, uint64_t ybase, void* stream) {
   if (!x || !w || !gate || !y || !fits31(rows) || !fits31(cols) || !(eps >= 0.0f)) return kInvalidArgument;
-  rmsnorm_gated_kernel<<<static_cast<unsigned>(rows), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      x, w, gate, y, static_cast<int>(cols), eps, gbase, ybase);
+  auto st = static_cast<cudaStream_t>(stream);
+  const unsigned n = static_cast<unsigned>(rows), ctas = (n + kHeadRows - 1) / kHeadRows;
+  if (cols == 128) rmsnorm_gated_heads_kernel<4><<<ctas, kHeadRows * 32, 0, st>>>(x, w, gate, y, n, eps, gbase, ybase);
+  else if (cols == 256) rmsnorm_gated_heads_kernel<8><<<ctas, kHeadRows * 32, 0, st>>>(x, w, gate, y, n, eps, gbase, ybase);
+  else rmsnorm_gated_kernel<<<n, 256, 0, st>>>(x, w, gate, y, static_cast<int>(cols), eps, gbase, ybase);
   return check_launch();
 }
 
@@ -573,6 +892,15 @@ int tsr_delta_step_heads(float* s, const float* k, const float* v, const float* 
   if (!s || !k || !v || !q || !o || !alpha || !beta || !fits31(heads) || !fits31(dk) || !fits31(dv) || !fits31(rows) ||
       dk > 256)
     return kInvalidArgument;
+  // One row is a pass over the state, which the general kernel reads in whole lines (a token's step over three layers was
+  // 1.8 us a layer slower here); it also serves heads of another width and vectors that are not 16-byte aligned.
+  if (rows >= 2 && dk == kDeltaDk && dv % kDeltaRowCols == 0 && aligned16(k) && aligned16(q) && aligned16(v)) {
+    delta_step_rows_kernel<<<static_cast<unsigned>(heads * (dv / kDeltaRowCols)), kDeltaRowThreads, 0,
+                             static_cast<cudaStream_t>(stream)>>>(s, k, v, q, o, alpha, beta, static_cast<int>(heads),
+                                                                  static_cast<int>(dv), static_cast<int>(rows), sbase, sstride,
+                                                                  abase);
+    return check_launch();
+  }
   const unsigned slabs = static_cast<unsigned>((dv + kDeltaCols - 1) / kDeltaCols);
   delta_step_heads_kernel<<<static_cast<unsigned>(heads) * slabs, kDeltaCols * kDeltaWarps, 0,
                             static_cast<cudaStream_t>(stream)>>>(s, k, v, q, o, alpha, beta, static_cast<int>(heads),
@@ -587,8 +915,13 @@ int tsr_conv1d_state(const float* qkv, const float* w, float* hist, float* q, fl
   if (!qkv || !w || !hist || !q || !k || !v || !fits31(conv_dim) || !fits31(width) || !fits31(rows) || 2 * key_dim > conv_dim ||
       (hist_stride != 0 && !hist_hist))
     return kInvalidArgument;
-  conv1d_state_kernel<<<blocks_of(conv_dim), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      qkv, w, hist, q, k, v, hist_hist, conv_dim, width, key_dim, qkv_offset, rows, hist_stride);
+  auto st = static_cast<cudaStream_t>(stream);
+  const dim3 grid(blocks_of(conv_dim), static_cast<unsigned>((rows + kConvRows - 1) / kConvRows));
+  if (width == 4 && grid.y <= 65535)  // the width of the convolutions in use; others take their rows in turn
+    conv1d_rows_kernel<4><<<grid, 256, 0, st>>>(qkv, w, hist, q, k, v, hist_hist, conv_dim, key_dim, qkv_offset, rows, hist_stride);
+  else
+    conv1d_state_kernel<<<blocks_of(conv_dim), 256, 0, st>>>(qkv, w, hist, q, k, v, hist_hist, conv_dim, width, key_dim,
+                                                             qkv_offset, rows, hist_stride);
   return check_launch();
 }
 
@@ -606,8 +939,13 @@ int tsr_repeat_heads(const float* in, float* out, uint64_t num_v_heads, uint64_t
       num_v_heads % factor != 0)
     return kInvalidArgument;
   const size_t total = rows * num_v_heads * head_k_dim;
-  repeat_heads_kernel<<<blocks_of(total), 256, 0, static_cast<cudaStream_t>(stream)>>>(in, out, num_v_heads, head_k_dim,
-                                                                                        num_v_heads / factor, total);
+  auto st = static_cast<cudaStream_t>(stream);
+  if (head_k_dim % 4 == 0 && total < (1ull << 31) && aligned16(in) && aligned16(out))
+    repeat_heads4_kernel<<<blocks_of(total / 4), 256, 0, st>>>(
+        reinterpret_cast<const float4*>(in), reinterpret_cast<float4*>(out), static_cast<unsigned>(num_v_heads),
+        static_cast<unsigned>(head_k_dim / 4), static_cast<unsigned>(num_v_heads / factor), static_cast<unsigned>(total / 4));
+  else
+    repeat_heads_kernel<<<blocks_of(total), 256, 0, st>>>(in, out, num_v_heads, head_k_dim, num_v_heads / factor, total);
   return check_launch();
 }
 

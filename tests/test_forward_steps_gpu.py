@@ -242,3 +242,33 @@ def test_top_k_rows(backend, oracle):
     lg = g.standard_normal(256).astype(np.float32)
     run(backend, "top_k_rows", [backend.upload(lg), ib, vb], [1, 256, 8, 0])
     assert np.array_equal(backend.download(ib, np.uint32, 8), np.argsort(-lg, kind="stable")[:8].astype(np.uint32))
+
+
+@pytest.mark.parametrize("heads,dv,rows,history", [(5, 48, 16, False), (2, 16, 33, True), (3, 128, 17, False), (2, 24, 5, False)])
+def test_delta_steps_over_blocks_of_rows(backend, oracle, heads, dv, rows, history):
+    """Whole and ragged blocks of 16 steps, the smallest slab of columns, and a width the row kernel leaves to the general one."""
+    test_delta_step_heads(backend, oracle, heads, 128, dv, rows, history)
+
+
+@pytest.mark.parametrize("rows,history", [(2, False), (16, True), (17, True), (33, False), (51, True)])
+def test_conv1d_over_chunks_of_rows(backend, oracle, rows, history):
+    """Fewer rows than the history holds, one chunk of 16 rows exactly, ragged later chunks."""
+    test_conv1d_state(backend, oracle, rows, history)
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 128), (9, 128), (9, 256), (17, 256)])
+def test_head_sized_rows(backend, oracle, rows, cols):
+    """A warp per row: the last CTA partly filled, both widths, in place (l2norm) and with element bases (rmsnorm_gated)."""
+    g = np.random.default_rng(rows * cols)
+    x = g.standard_normal((rows, cols)).astype(np.float32)
+    xb = backend.upload(x)
+    run(backend, "l2norm", [xb, xb], [rows, cols, bits(1e-6), bits(0.25)])
+    want = oracle.l2norm(x, 1e-6, np.float32(0.25))
+    assert close(backend.download(xb, np.float32, rows * cols), want.reshape(-1), 2e-6)
+    w, gate = g.standard_normal(cols).astype(np.float32), g.standard_normal((rows, cols)).astype(np.float32)
+    yb = backend.upload(np.full(rows * cols + 7, np.float32(-3e9)))
+    gb = backend.upload(np.concatenate([np.zeros(5, np.float32), gate.reshape(-1)]))
+    run(backend, "rmsnorm_gated", [backend.upload(x), backend.upload(w), gb, yb], [rows, cols, bits(1e-6), 5, 3])
+    y = backend.download(yb, np.float32, rows * cols + 7)
+    assert close(y[3:-4], oracle.rmsnorm_gated(x, w, gate, 1e-6).reshape(-1), 2e-6)
+    assert np.all(y[:3] == np.float32(-3e9)) and np.all(y[-4:] == np.float32(-3e9))
