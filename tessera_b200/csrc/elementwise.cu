@@ -163,6 +163,23 @@ __global__ void silu_mul_kernel(const float* __restrict__ g, const float* __rest
   o[idx] = x / (1.0f + expf(-x)) * u[idx];
 }
 
+// The same and `add`, sixteen bytes a load (n a multiple of four, 16-byte aligned buffers): an element a thread kept too
+// few bytes in flight for a prompt chunk (512 x 17408: silu_mul 40 us, here 17 us, 107 MB at 6.3 TB/s).
+__global__ void __launch_bounds__(256) silu_mul4_kernel(const float4* g, const float4* u,
+                                                        float4* o, size_t n4) {
+  const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= n4) return;
+  const float4 x = g[i], y = u[i];
+  o[i] = make_float4(x.x / (1.0f + expf(-x.x)) * y.x, x.y / (1.0f + expf(-x.y)) * y.y, x.z / (1.0f + expf(-x.z)) * y.z,
+                     x.w / (1.0f + expf(-x.w)) * y.w);
+}
+__global__ void __launch_bounds__(256) add4_kernel(const float4* a, const float4* b, float4* o, size_t n4) {
+  const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= n4) return;
+  const float4 x = a[i], y = b[i];
+  o[i] = make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w);
+}
+
 // Y = X / sqrt(mean(X^2) + eps) * W, one CTA per row (RmsNormRef, src/core/numerics/norm.cpp:7-32;
 // the reference adds the squares sequentially, here they are added as a tree).
 __global__ void __launch_bounds__(1024)
@@ -187,6 +204,14 @@ rmsnorm_kernel(const float* __restrict__ x, const float* __restrict__ w, float* 
   for (int c = threadIdx.x; c < cols; c += blockDim.x) out[c] = row[c] * gain * w[c];
 }
 
+// Whether an elementwise step over n floats takes the four-wide kernel: from 64k elements on (below, a quarter of the
+// threads is a quarter of the SMs), whole and aligned, and with an output that is one of the inputs or apart from them (a
+// thread reads four elements before it writes four).
+static bool wide4(const float* a, const float* b, const float* o, uint64_t n) {
+  auto apart = [&](const float* x) { return x == o || o + n <= x || x + n <= o; };
+  return n >= (1u << 16) && n % 4 == 0 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(o)) & 15u) == 0 &&
+         apart(a) && apart(b);
+}
 static unsigned blocks_for(uint64_t n, unsigned per) {
   return static_cast<unsigned>((n + per - 1) / per);
 }
@@ -242,13 +267,23 @@ int tsr_round_bf16(float* x, uint64_t n, void* stream) {
 
 int tsr_add(const float* a, const float* b, float* o, uint64_t n, void* stream) {
   if (!a || !b || !o || n == 0) return kInvalidArgument;
+  if (wide4(a, b, o, n)) {
+    add4_kernel<<<blocks_for(n / 4, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        reinterpret_cast<const float4*>(a), reinterpret_cast<const float4*>(b), reinterpret_cast<float4*>(o), n / 4);
+    return check_launch();
+  }
   add_kernel<<<blocks_for(n, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(a, b, o, n);
   return check_launch();
 }
 
 int tsr_silu_mul(const float* g, const float* u, float* o, uint64_t n, void* stream) {
   if (!g || !u || !o || n == 0) return kInvalidArgument;
-  silu_mul_kernel<<<blocks_for(n, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(g, u, o, n);
+  auto st = static_cast<cudaStream_t>(stream);
+  if (wide4(g, u, o, n))
+    silu_mul4_kernel<<<blocks_for(n / 4, 256), 256, 0, st>>>(reinterpret_cast<const float4*>(g), reinterpret_cast<const float4*>(u),
+                                                             reinterpret_cast<float4*>(o), n / 4);
+  else
+    silu_mul_kernel<<<blocks_for(n, 256), 256, 0, st>>>(g, u, o, n);
   return check_launch();
 }
 
