@@ -11,15 +11,13 @@
 // reference's own tensor-core tile does (src/backends/rocm/rocm_kernels_wmma.cpp:
 // 54-80 of the reference: weights dequantised to fp16 in shared memory).
 //
-// Per CTA: four producer warps (thread = weight row; the operand-B pieces are
-// shared out among all 128 threads) dequantise a 64-wide k slab, from raw
-// bytes loaded four slabs ahead, into the canonical K-major no-swizzle UMMA
-// layout (8x16-byte core matrices; leading-byte offset 128 B along k, stride
-// byte offset 1024 B along rows), fence it to the async proxy and signal a
-// full barrier; one elected thread issues four K=16 MMAs per slab and commits
-// them to the slab's empty barrier; two slab buffers overlap dequantisation
-// with the MMAs.  The producer warps then read the accumulator with tcgen05.ld
-// (warp w owns TMEM lanes 32*(w%4)..), add the hi and lo columns and store C.
+// Two kernels.  gemm_umma_ring_kernel (below the ring) takes weights that TMA can fetch and activations that were
+// converted ahead, which is nearly every launch.  gemm_umma_kernel takes the rest (k not a whole number of ring
+// segments, unaligned weights, no scratch): eight producer warps, two threads per weight row, dequantise a 64-wide k
+// slab into the canonical K-major no-swizzle UMMA layout (8x16-byte core matrices; leading-byte offset 128 B along k,
+// stride byte offset 1024 B along rows), fence it to the async proxy and signal a full barrier; one elected thread
+// issues four K=16 MMAs per slab and commits them to the slab's empty barrier.  The producer warps then read the
+// accumulator with tcgen05.ld (warp w owns TMEM lanes 32*(w%4)..), add the hi and lo columns and store C.
 // Every wait is bounded and TMEM is always released.
 #include <cuda_fp16.h>
 
@@ -47,8 +45,8 @@ constexpr int kProducerThreads = 256;  // two per weight row
 constexpr int kUmmaThreads = kProducerThreads + 96;  // + the MMA warp, the weight TMA warp, the activation copy warp
 constexpr int kBSlabPitch = 512 * kSlab * 2;  // bytes per slab of pre-converted activations: up to 512 operand rows (64 KiB)
 constexpr int kASlabBytes = kTileM * kSlab * 2;  // 16384
-constexpr int kBufs = 2;                         // slab buffers in shared memory (a power of two)
-constexpr int kBufShift = 1;
+constexpr int kBufs = 2;                         // slab buffers when the producers fill operand B too
+constexpr int kMaxABufs = 6, kMaxBBufs = 4, kMaxRaw = 4;  // most buffers of weight slabs, activation slabs, raw stages
 constexpr uint32_t kLbo = 128, kSbo = (kSlab / 8) * 128;  // bytes
 
 enum Format { kFmtQ4K = 0, kFmtQ6K = 1, kFmtMxFp4 = 2, kFmtFp8 = 3 };
@@ -62,6 +60,8 @@ struct UmmaParams {
   const unsigned char* bpre;  // activations already in operand layout (convert_activations_kernel), or null
   int split_slabs;            // k is cut among gridDim.z CTAs, this many 64-wide slabs each (a multiple of a ring
                               // stage); CTA z writes its partial sums to region z of c (m x n floats each)
+  int a_bufs, b_bufs, raw_stages;  // buffers of each kind in this launch's shared memory
+  int issuers, by_columns;         // MMA issuers of the ring kernel; whether they share every slab's columns or take slabs in turn
   int one_term;               // batches beyond one chunk: a single binary16 term per activation; 1: 128 tokens per
                               // CTA, 2: 256, 3: 512 as two accumulators of 256 columns (2 and 3 need the
                               // pre-converted activations)
@@ -220,9 +220,10 @@ __device__ __forceinline__ void convert(const UmmaParams& p, int row, int slab, 
   if (FMT == kFmtQ4K) {
     const int sb = 2 * (slab & 3) + half;  // sub-block: low nibbles are the even one
     const float d = fp16_bits_to_float(r.x[0] & 0xFFFFu), dmin = fp16_bits_to_float(r.x[0] >> 16);
-    const uint32_t s[3] = {r.x[1], r.x[2], r.x[3]};
-    uint32_t sc, mn;
-    q4k_scale_min(s, sb, sc, mn);
+    // pair sb of the 12 packed bytes (q4k_scale_min) by shifts: indexing the words by sb put them in local memory
+    const uint32_t s0 = r.x[1] >> (8 * (sb & 3)), s1 = r.x[2] >> (8 * (sb & 3)), s2 = r.x[3] >> (8 * (sb & 3));
+    const uint32_t sc = sb < 4 ? s0 & 63u : (s2 & 15u) | ((s0 >> 2) & 48u);
+    const uint32_t mn = sb < 4 ? s1 & 63u : ((s2 >> 4) & 15u) | ((s1 >> 2) & 48u);
     const uint32_t dl = h2_const(d * static_cast<float>(sc)), ml = h2_const(-dmin * static_cast<float>(mn));
     const uint32_t qw[8] = {r.q[0].x, r.q[0].y, r.q[0].z, r.q[0].w, r.q[1].x, r.q[1].y, r.q[1].z, r.q[1].w};
 #pragma unroll
@@ -298,11 +299,12 @@ __device__ __forceinline__ uint4 convert_b_piece(float4 x0, float4 x1, bool lo_p
 // tiles fetch a slab with one bulk copy instead of converting it in every CTA.
 __global__ void __launch_bounds__(256)
 convert_activations_kernel(const float* __restrict__ a, unsigned char* __restrict__ out, int m, int k, int one_term) {
+  // gridDim.z CTAs share a slab
   const int slab = blockIdx.x, chunk = blockIdx.y, nslabs = gridDim.x;
   const TokenChunk tc = token_chunk(m, chunk, one_term);
   const int tok0 = tc.tok0, tokens = tc.tokens, tok_pad = tc.tok_pad, n_cols = 2 * tok_pad;
   unsigned char* dst = out + (static_cast<size_t>(chunk) * nslabs + slab) * kBSlabPitch;
-  for (int g = threadIdx.x; g < n_cols * (kSlab / 8); g += blockDim.x) {
+  for (int g = blockIdx.z * blockDim.x + threadIdx.x; g < n_cols * (kSlab / 8); g += gridDim.z * blockDim.x) {
     const int r = g >> 3, kc = g & 7;
     bool lo_part;
     const int tok = row_token(r, tok_pad, one_term, &lo_part);
@@ -317,20 +319,25 @@ convert_activations_kernel(const float* __restrict__ a, unsigned char* __restric
 
 // ---- raw-weight ring (TMA) ------------------------------------------------------
 // With RING the weight bytes of a 128-row tile arrive by tiled TMA copies, a
-// stage of several slabs at a time, in a ring of kRawStages stages; the
+// stage of several slabs at a time, in a ring of two to four stages; the
 // producers read their 16-byte pieces from shared memory.  Per-thread global
 // loads (thread = row) touch 32 different lines per warp instruction and ran
 // at an eighth of the memory rate.  Stage layouts:
 //   FP8   [2 segments][128 rows][128 B], 128-byte swizzle       (256 k, 4 slabs)
 //   MXFP4 the same for the nibbles (512 k, 8 slabs) + [128 rows][16 scale bytes]
 //   Q4_K  [128 rows][144 B]: one block per row                  (256 k, 4 slabs)
-// Q6_K (2-byte aligned blocks) and shapes whose k is not a whole number of
-// segments keep the direct loads (RING = false).
-constexpr int kRawStages = 3;
+// Q6_K with another k (2-byte aligned blocks) and shapes whose k is not a whole number
+// of segments keep the direct loads (RING = false).
+//   Q6_K  [64 even rows][240 B], [64 odd rows][240 B]: a block per row (256 k, 4 slabs).  Rows of 210-byte blocks are
+//         8-byte aligned when k/256 is a multiple of 4, and a copy wants 16: the even and the odd rows are two tensors
+//         with a pitch of two rows, the odd one based at the 16-byte boundary below its first row.  A box starts at the
+//         boundary below the block and holds it whole (up to 14 bytes in front of it); 240 bytes a row keep the
+//         producers' 16-byte reads conflict-free (60 = 28 mod 32 words).
+constexpr int kQ6KPitch = 240;
 template <int FMT>
 struct RingFmt {
   static constexpr int kSlabsPerStage = FMT == kFmtMxFp4 ? 8 : 4;
-  static constexpr int kWeightBytes = FMT == kFmtQ4K ? kTileM * kQ4KBlockBytes : 2 * kTileM * 128;
+  static constexpr int kWeightBytes = FMT == kFmtQ4K ? kTileM * kQ4KBlockBytes : FMT == kFmtQ6K ? kTileM * kQ6KPitch : 2 * kTileM * 128;
   static constexpr int kScaleBytes = FMT == kFmtMxFp4 ? kTileM * 16 : 0;
   static constexpr int kStageBytes = kWeightBytes + kScaleBytes;
   static constexpr int kStagePitch = (kStageBytes + 1023) & ~1023;  // stages start on 1 KiB boundaries (swizzle)
@@ -355,6 +362,67 @@ __device__ __forceinline__ void read_raw(const unsigned char* stage, int trow, i
   }
 }
 
+// The TMA copies of one raw stage: stage `sta` of the whole k, rows from row0.
+template <int FMT>
+__device__ __forceinline__ void load_raw_stage(const CUtensorMap& wmap, const CUtensorMap& smap, unsigned char* dst, int k,
+                                               int row0, int sta, uint64_t* bar) {
+  mbar_expect_tx(bar, RingFmt<FMT>::kStageBytes);
+  if (FMT == kFmtQ4K) {
+    tma_load_3d(dst, &wmap, 0, sta, row0, bar);  // (18 x u64, block, rows)
+  } else if (FMT == kFmtQ6K) {
+    // (30 x u64, row pairs): the 16-byte boundary below the block, even then odd rows
+    const int odd = (k / 256 * kQ6KBlockBytes) & 15, at = sta * kQ6KBlockBytes;
+    tma_load_2d(dst, &wmap, (at & ~15) / 8, row0 / 2, bar);
+    tma_load_2d(dst + (kTileM / 2) * kQ6KPitch, &smap, ((at + odd) & ~15) / 8, row0 / 2, bar);
+  } else {
+    tma_load_3d(dst, &wmap, 0, row0, 2 * sta, bar);  // (128 B, rows, segments)
+    if (FMT == kFmtMxFp4) tma_load_2d(dst + RingFmt<FMT>::kWeightBytes, &smap, 16 * sta, row0, bar);
+  }
+}
+
+// 32 bytes that start `rem` (even, below 16) bytes into `p` (16-byte aligned), as words.  rem is the same for a whole warp.
+__device__ __forceinline__ void load_shifted32(const unsigned char* p, int rem, uint32_t (&o)[8]) {
+  const uint4 x = *reinterpret_cast<const uint4*>(p), y = *reinterpret_cast<const uint4*>(p + 16),
+              z = *reinterpret_cast<const uint4*>(p + 32);
+  uint32_t w[12] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w, z.x, z.y, z.z, z.w};
+  if (rem & 8) {
+#pragma unroll
+    for (int i = 0; i < 10; ++i) w[i] = w[i + 2];
+  }
+  if (rem & 4) {
+#pragma unroll
+    for (int i = 0; i < 9; ++i) w[i] = w[i + 1];
+  }
+  const uint32_t sh = (rem & 2) * 8;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) o[i] = __funnelshift_r(w[i], w[i + 1], sh);
+}
+// Half a slab (32 weights) of a Q6_K block that lies `rem` bytes into its row of a raw stage; the arithmetic of
+// convert<kFmtQ6K>: the fp32 product of d * scale and q - 32, rounded to binary16 once.
+__device__ __forceinline__ void convert_q6k_stage(const unsigned char* row, int rem, int j, int half, uint4 (&out)[4]) {
+  const int hh = j >> 1, pp = 2 * (j & 1) + half;
+  uint32_t ql[8], qh[8];
+  load_shifted32(row + 64 * hh + 32 * half, rem, ql);
+  load_shifted32(row + 128 + 32 * hh, rem, qh);
+  const float d = fp16_bits_to_float(*reinterpret_cast<const unsigned short*>(row + rem + 208));
+  const uint32_t scw = *reinterpret_cast<const unsigned short*>(row + rem + 192 + 8 * hh + 2 * pp);
+  const float s[2] = {d * static_cast<float>(static_cast<signed char>(scw & 0xFFu)),
+                      d * static_cast<float>(static_cast<signed char>(scw >> 8))};
+  uint32_t h[16];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const uint32_t q = ((ql[i] >> (2 * (pp & 2))) & 0x0F0F0F0Fu) | (((qh[i] >> (2 * pp)) & 0x03030303u) << 4);
+    float v[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)  // the byte into the low mantissa bits of 2^23, exact
+      v[e] = s[i >> 2] * (__uint_as_float(__byte_perm(q, 0x4B000000u, 0x7540 + e)) - (8388608.0f + 32.0f));
+    h[2 * i] = pack_h2(v[0], v[1]);
+    h[2 * i + 1] = pack_h2(v[2], v[3]);
+  }
+#pragma unroll
+  for (int kc = 0; kc < 4; ++kc) out[kc] = make_uint4(h[4 * kc], h[4 * kc + 1], h[4 * kc + 2], h[4 * kc + 3]);
+}
+
 template <int FMT, bool RING>
 __global__ void __launch_bounds__(kUmmaThreads)
 gemm_umma_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap smap,
@@ -368,18 +436,19 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
   const int tok_pad = tc.tok_pad;             // rows [0, tok_pad) and [tok_pad, 2*tok_pad): see token_chunk
   const int n_cols = 2 * tok_pad;             // multiple of 16, <= 128
   const int b_slab_bytes = n_cols * kSlab * 2;
-  constexpr int kRingBytes = RING ? kRawStages * RingFmt<FMT>::kStagePitch : 0;
-  unsigned char* const ring = smem;                            // [kRawStages][kStagePitch]
-  unsigned char* const a_tiles = smem + kRingBytes;            // [kBufs][kASlabBytes]
-  unsigned char* const b_tiles = a_tiles + kBufs * kASlabBytes;  // [kBufs][b_slab_bytes]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(b_tiles + kBufs * b_slab_bytes);
-  uint64_t* full = bars;                 // [kBufs] producers -> MMA
-  uint64_t* empty = bars + kBufs;        // [kBufs] MMA -> producers
-  uint64_t* done = bars + 2 * kBufs;     // accumulator complete
-  uint64_t* raw_full = done + 1;         // [kRawStages] TMA -> producers
-  uint64_t* raw_empty = raw_full + kRawStages;  // [kRawStages] producers -> TMA
-  uint64_t* b_full = raw_empty + kRawStages;    // [kBufs] activation copy -> MMA
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(b_full + kBufs);
+  const int ring_bytes = RING ? p.raw_stages * RingFmt<FMT>::kStagePitch : 0;
+  unsigned char* const ring = smem;                                 // [raw_stages][kStagePitch]
+  unsigned char* const a_tiles = smem + ring_bytes;                 // [a_bufs][kASlabBytes]
+  unsigned char* const b_tiles = a_tiles + p.a_bufs * kASlabBytes;  // [b_bufs][b_slab_bytes]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(b_tiles + p.b_bufs * b_slab_bytes);
+  uint64_t* full = bars;                     // [a_bufs] producers -> MMA
+  uint64_t* empty = full + kMaxABufs;        // [a_bufs] MMA -> producers
+  uint64_t* done = empty + kMaxABufs;        // accumulator complete
+  uint64_t* raw_full = done + 1;             // [raw_stages] TMA -> producers
+  uint64_t* raw_empty = raw_full + kMaxRaw;  // [raw_stages] producers -> TMA
+  uint64_t* b_full = raw_empty + kMaxRaw;    // [b_bufs] activation copy -> MMA
+  uint64_t* b_empty = b_full + kMaxBBufs;    // [b_bufs] MMA -> activation copy
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(b_empty + kMaxBBufs);
   uint32_t tmem_cols = 32;
   while (tmem_cols < static_cast<uint32_t>(n_cols)) tmem_cols <<= 1;
   const int total_slabs = p.k / kSlab;
@@ -388,12 +457,15 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
   constexpr int kProducerWarps = kProducerThreads / 32;  // then the MMA warp, the weight TMA warp, the activation copy warp
 
   if (tid == 0) {
-    for (int s = 0; s < kBufs; ++s) {
+    for (int s = 0; s < p.a_bufs; ++s) {
       mbar_init(&full[s], kProducerThreads / 32);  // one arrival per producer warp
       mbar_init(&empty[s], 1);
-      mbar_init(&b_full[s], 1);
     }
-    for (int s = 0; s < kRawStages; ++s) {
+    for (int s = 0; s < p.b_bufs; ++s) {
+      mbar_init(&b_full[s], 1);
+      mbar_init(&b_empty[s], 1);
+    }
+    for (int s = 0; s < p.raw_stages; ++s) {
       mbar_init(&raw_full[s], 1);
       mbar_init(&raw_empty[s], kProducerThreads / 32);
     }
@@ -409,8 +481,14 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
 
   if (warp < kProducerWarps) {
     // ---------------- producers: dequantise A rows, convert B rows ---------
-    const int trow = tid & (kTileM - 1), half = tid >> 7;  // warps 0-3: first 32 k of a slab, warps 4-7: the rest
+    // warps 0-3: first 32 k of a slab, warps 4-7: the rest.  slot_row: the thread's row of a raw stage; Q6_K stages hold
+    // the even rows, then the odd ones (so that a warp's rows share the block's offset in its box)
+    const int slot_row = tid & (kTileM - 1), half = tid >> 7;
+    const int trow = FMT == kFmtQ6K && RING ? ((slot_row & 63) << 1) | (slot_row >> 6) : slot_row;
     const int wrow = row0 + trow;
+    // offset of block b of a row in its box: 210 b = 2 b mod 16, the odd rows' base lies (210 k/256) mod 16 below them
+    const int odd_base = (slot_row >> 6) * ((p.k / 256 * kQ6KBlockBytes) & 15);
+    auto q6k_rem = [&](int b) { return (2 * b + odd_base) & 15; };
     const bool have_row = wrow < p.n;
     // Without the ring: raw bytes by direct loads, a group of kAhead slabs at a time, one group ahead.
     constexpr int kAhead = 4;
@@ -453,48 +531,13 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
       load_b(0, bx[0]);
       load_b(1, bx[1]);
     }
-    if (RING && !convert_b) {
-      // The common case (weights from the ring, activations from the scratch copy) as one
-      // rolled loop: nothing here lives in per-slab registers, and the unrolled form
-      // below spent a fifth of its issue slots waiting for instruction fetch.
-#pragma unroll 1
-      for (int s = 0; s < nslabs; ++s) {
-        const int buf = s & (kBufs - 1), round = s >> kBufShift;
-        if (round > 0 && !mbar_wait(&empty[buf], (round - 1) & 1, &g_umma_timeouts)) {
-          failed = true;
-          break;
-        }
-        constexpr int kPer = RingFmt<FMT>::kSlabsPerStage;
-        const int st = s / kPer, si = s - st * kPer;
-        const int slot = st % kRawStages, rround = st / kRawStages;
-        if (si == 0 && !mbar_wait(&raw_full[slot], rround & 1, &g_umma_timeouts)) {
-          failed = true;
-          break;
-        }
-        uint4 piece4[4] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u),
-                           make_uint4(0u, 0u, 0u, 0u)};
-        RawHalf rr;
-        read_raw<FMT>(ring + slot * RingFmt<FMT>::kStagePitch, trow, si, half, rr);
-        if (have_row) convert<FMT>(p, wrow, s_off + s, half, rr, piece4);
-        if (si == kPer - 1 || s == nslabs - 1) {  // this warp is done with the stage
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&raw_empty[slot]);
-        }
-        unsigned char* a_dst = a_tiles + buf * kASlabBytes + (trow >> 3) * kSbo + (trow & 7) * 16 + half * 4 * kLbo;
-#pragma unroll
-        for (int kc = 0; kc < 4; ++kc) *reinterpret_cast<uint4*>(a_dst + kc * kLbo) = piece4[kc];
-        fence_async_proxy();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&full[buf]);
-      }
-    } else
     for (int s0 = 0; s0 < nslabs && !failed; s0 += 2 * kAhead) {
 #pragma unroll
       for (int uu = 0; uu < 2 * kAhead; ++uu) {
         const int grp = uu / kAhead, u = uu % kAhead;
         const int s = s0 + uu;
         if (s >= nslabs || failed) break;
-        const int buf = s & (kBufs - 1), round = s >> kBufShift;
+        const int buf = s % p.a_bufs, round = s / p.a_bufs;
         if (round > 0 && !mbar_wait(&empty[buf], (round - 1) & 1, &g_umma_timeouts)) {
           failed = true;
           break;
@@ -504,14 +547,19 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
         if (RING) {
           constexpr int kPer = RingFmt<FMT>::kSlabsPerStage;
           const int st = s / kPer, si = s - st * kPer;
-          const int slot = st % kRawStages, rround = st / kRawStages;
+          const int slot = st % p.raw_stages, rround = st / p.raw_stages;
           if (si == 0 && !mbar_wait(&raw_full[slot], rround & 1, &g_umma_timeouts)) {
             failed = true;
             break;
           }
-          RawHalf rr;
-          read_raw<FMT>(ring + slot * RingFmt<FMT>::kStagePitch, trow, si, half, rr);
-          if (have_row) convert<FMT>(p, wrow, s_off + s, half, rr, piece4);
+          const unsigned char* stage = ring + slot * RingFmt<FMT>::kStagePitch;
+          if constexpr (FMT == kFmtQ6K) {
+            if (have_row) convert_q6k_stage(stage + slot_row * kQ6KPitch, q6k_rem((s_off + s) / kPer), si, half, piece4);
+          } else {
+            RawHalf rr;
+            read_raw<FMT>(stage, trow, si, half, rr);
+            if (have_row) convert<FMT>(p, wrow, s_off + s, half, rr, piece4);
+          }
           if (si == kPer - 1 || s == nslabs - 1) {  // this warp is done with the stage
             __syncwarp();
             if (lane == 0) mbar_arrive(&raw_empty[slot]);
@@ -551,15 +599,15 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
       const int n_first = n_cols > 256 ? 256 : n_cols, n_second = n_cols - n_first;
       const uint32_t idesc = instr_desc(static_cast<uint32_t>(n_first));
       const uint32_t idesc2 = instr_desc(static_cast<uint32_t>(n_second > 0 ? n_second : 16));
+      int buf = 0, round = 0, bbuf = 0, bround = 0;  // operand B has buffers of its own when it is copied in
       for (int s = 0; s < nslabs; ++s) {
-        const int buf = s & (kBufs - 1), round = s >> kBufShift;
         if (!mbar_wait(&full[buf], round & 1, &g_umma_timeouts) ||
-            (p.bpre != nullptr && !mbar_wait(&b_full[buf], round & 1, &g_umma_timeouts))) {
+            (p.bpre != nullptr && !mbar_wait(&b_full[bbuf], bround & 1, &g_umma_timeouts))) {
           failed = true;
           break;
         }
         tcgen05_fence_after();
-        const uint32_t a_addr = smem_u32(a_tiles + buf * kASlabBytes), b_addr = smem_u32(b_tiles + buf * b_slab_bytes);
+        const uint32_t a_addr = smem_u32(a_tiles + buf * kASlabBytes), b_addr = smem_u32(b_tiles + bbuf * b_slab_bytes);
 #pragma unroll
         for (int kk = 0; kk < kSlab / 16; ++kk) {
           umma_f16(tmem_base, smem_desc(a_addr + kk * 2 * kLbo), smem_desc(b_addr + kk * 2 * kLbo), idesc,
@@ -568,7 +616,10 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
             umma_f16(tmem_base + 256, smem_desc(a_addr + kk * 2 * kLbo), smem_desc(b_addr + (256 / 8) * kSbo + kk * 2 * kLbo),
                      idesc2, (s > 0 || kk > 0) ? 1u : 0u);
         }
-        umma_commit(&empty[buf]);  // the slab buffer is free once these MMAs have read it
+        umma_commit(&empty[buf]);  // the slab buffers are free once these MMAs have read them
+        if (p.bpre != nullptr) umma_commit(&b_empty[bbuf]);
+        if (++buf == p.a_bufs) buf = 0, ++round;
+        if (++bbuf == p.b_bufs) bbuf = 0, ++bround;
       }
       umma_commit(done);
     }
@@ -577,17 +628,9 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
     constexpr int kPer = RingFmt<FMT>::kSlabsPerStage;
     const int nstages = (nslabs + kPer - 1) / kPer;
     for (int st = 0; st < nstages; ++st) {
-      const int slot = st % kRawStages, rround = st / kRawStages;
+      const int slot = st % p.raw_stages, rround = st / p.raw_stages;
       if (rround > 0 && !mbar_wait(&raw_empty[slot], (rround - 1) & 1, &g_umma_timeouts)) break;
-      unsigned char* dst = ring + slot * RingFmt<FMT>::kStagePitch;
-      mbar_expect_tx(&raw_full[slot], RingFmt<FMT>::kStageBytes);
-      const int sta = s_off / kPer + st;  // the stage's index in the whole k
-      if (FMT == kFmtQ4K) {
-        tma_load_3d(dst, &wmap, 0, sta, row0, &raw_full[slot]);      // (18 x u64, block, rows)
-      } else {
-        tma_load_3d(dst, &wmap, 0, row0, 2 * sta, &raw_full[slot]);  // (128 B, rows, segments)
-        if (FMT == kFmtMxFp4) tma_load_2d(dst + RingFmt<FMT>::kWeightBytes, &smap, 16 * sta, row0, &raw_full[slot]);
-      }
+      load_raw_stage<FMT>(wmap, smap, ring + slot * RingFmt<FMT>::kStagePitch, p.k, row0, s_off / kPer + st, &raw_full[slot]);
     }
   }
 
@@ -595,8 +638,8 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
     // ---------------- activation copy: one bulk copy per slab ----------------
     const unsigned char* src = p.bpre + (static_cast<size_t>(blockIdx.y) * total_slabs + s_off) * kBSlabPitch;
     for (int s = 0; s < nslabs; ++s) {
-      const int buf = s & (kBufs - 1), round = s >> kBufShift;
-      if (round > 0 && !mbar_wait(&empty[buf], (round - 1) & 1, &g_umma_timeouts)) break;
+      const int buf = s % p.b_bufs, round = s / p.b_bufs;
+      if (round > 0 && !mbar_wait(&b_empty[buf], (round - 1) & 1, &g_umma_timeouts)) break;
       mbar_expect_tx(&b_full[buf], static_cast<uint32_t>(b_slab_bytes));
       bulk_load(b_tiles + buf * b_slab_bytes, src + static_cast<size_t>(s) * kBSlabPitch,
                 static_cast<uint32_t>(b_slab_bytes), &b_full[buf]);
@@ -642,6 +685,264 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
   if (warp == kProducerWarps) tmem_dealloc(tmem_base, tmem_cols);
 }
 
+// ---- the tile for weights from the ring and activations converted ahead ------------------
+// The common case, every warp with one job:
+//   kRingGroups groups of eight producer warps, group g dequantises slabs g, g + kRingGroups, ... (two threads per
+//     weight row; BATCH slabs at a time with one proxy fence for them),
+//   up to four MMA issuers, one warp each for the raw-weight TMA and the activation copies.
+// Weight slabs, activation slabs and raw stages have rings of their own (a_bufs, b_bufs, raw_stages).
+// What bounds it.  Below 512 columns: the instructions of the thread that issues the MMAs.  A slab costs that thread
+// about 1200 cycles (two waits of 230, 480 to 540 for four or eight MMAs, two commits) against 260 (128 columns) to 1050
+// (512) cycles of the tensor pipe, and more producers or deeper rings changed nothing.  So the slabs of up to 256 columns
+// go round two issuers and those of up to 128 columns round four, each with an accumulator of its own that the epilogue
+// adds in order (shorter chains also round less: MXFP4 at 64 rows 3.5e-6 -> 4.5e-7 against 64 bits).  At 512 columns
+// (shared by two issuers): shared memory, which takes 64 KB of activations a slab in and gives them out once.
+// Measured, 17408 x 5120, one launch: 64 columns x two terms 55 -> 41 us (Q4_K), 56 -> 34 (MXFP4); 256 tokens 115 -> 63;
+// 512 tokens 91 -> 84; Q6_K 5120 x 17408 at 512 tokens 233 -> 98 us (its blocks came by 16-bit loads before).
+constexpr int kRingGroups = 2;
+constexpr int kRingProducerWarps = kRingGroups * kProducerThreads / 32;
+constexpr int kMaxIssuers = 4;
+constexpr int kRingTmaWarp = kRingProducerWarps + kMaxIssuers, kRingCopyWarp = kRingTmaWarp + 1;
+constexpr int kRingThreads = (kRingCopyWarp + 1) * 32;
+
+template <int FMT, int BATCH>
+__global__ void __launch_bounds__(kRingThreads, 1)
+gemm_umma_ring_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap smap,
+                      const UmmaParams p) {
+  using R = RingFmt<FMT>;
+  constexpr int kPer = R::kSlabsPerStage;
+  static_assert(kPer % (kRingGroups * BATCH) == 0, "a group's batches lie within a stage");
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int row0 = blockIdx.x * kTileM;
+  const TokenChunk tc = token_chunk(p.m, blockIdx.y, p.one_term);
+  const int n_cols = 2 * tc.tok_pad;
+  const int b_slab_bytes = n_cols * kSlab * 2;
+  unsigned char* const ring = smem;                                       // [raw_stages][kStagePitch]
+  unsigned char* const a_tiles = smem + p.raw_stages * R::kStagePitch;    // [a_bufs][kASlabBytes]
+  unsigned char* const b_tiles = a_tiles + p.a_bufs * kASlabBytes;        // [b_bufs][b_slab_bytes]
+  uint64_t* full = reinterpret_cast<uint64_t*>(b_tiles + p.b_bufs * b_slab_bytes);  // [a_bufs] producers -> MMA
+  uint64_t* empty = full + kMaxABufs;        // [a_bufs] MMA -> producers
+  uint64_t* done = empty + kMaxABufs;        // accumulator complete
+  uint64_t* raw_full = done + 1;             // [raw_stages] TMA -> producers
+  uint64_t* raw_empty = raw_full + kMaxRaw;  // [raw_stages] producers -> TMA
+  uint64_t* b_full = raw_empty + kMaxRaw;    // [b_bufs] activation copy -> MMA
+  uint64_t* b_empty = b_full + kMaxBBufs;    // [b_bufs] MMA -> activation copy
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(b_empty + kMaxBBufs);
+  const int total_slabs = p.k / kSlab;
+  const int s_off = gridDim.z > 1 ? static_cast<int>(blockIdx.z) * p.split_slabs : 0;  // this CTA's first slab
+  const int nslabs = gridDim.z > 1 ? min(p.split_slabs, total_slabs - s_off) : total_slabs;
+  const bool by_columns = p.by_columns != 0;
+  const int issuers = by_columns ? p.issuers : min(p.issuers, nslabs);
+  const int acc_cols = by_columns ? 256 : (n_cols + 31) & ~31;  // accumulator g starts at column g acc_cols
+  uint32_t tmem_cols = 32;
+  while (tmem_cols < static_cast<uint32_t>(issuers * acc_cols)) tmem_cols <<= 1;
+
+  if (tid == 0) {
+    for (int s = 0; s < p.a_bufs; ++s) {
+      mbar_init(&full[s], kProducerThreads / 32);  // one arrival per warp of the slab's group
+      mbar_init(&empty[s], by_columns ? 2 : 1);
+    }
+    for (int s = 0; s < p.b_bufs; ++s) {
+      mbar_init(&b_full[s], 1);
+      mbar_init(&b_empty[s], by_columns ? 2 : 1);
+    }
+    for (int s = 0; s < p.raw_stages; ++s) {
+      mbar_init(&raw_full[s], 1);
+      mbar_init(&raw_empty[s], kRingProducerWarps);
+    }
+    mbar_init(done, issuers);
+    mbar_fence_init();
+  }
+  if (warp == kRingProducerWarps) tmem_alloc(tmem_slot, tmem_cols);
+  tcgen05_fence_before();
+  __syncthreads();
+  tcgen05_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  bool failed = false;
+
+  if (warp < kRingProducerWarps) {
+    // ---------------- producers ---------------------------------------------
+    const int group = tid / kProducerThreads;
+    // a group's first four warps: the first 32 k of a slab, the others: the rest.  slot_row: the thread's row of a raw
+    // stage; Q6_K stages hold the even rows, then the odd ones (so that a warp's rows share the block's offset in its box)
+    const int slot_row = tid & (kTileM - 1), half = (tid >> 7) & 1;
+    const int trow = FMT == kFmtQ6K ? ((slot_row & 63) << 1) | (slot_row >> 6) : slot_row;
+    const int wrow = row0 + trow;
+    const bool have_row = wrow < p.n;
+    // offset of block b of a row in its box: 210 b = 2 b mod 16, the odd rows' base lies (210 k/256) mod 16 below them
+    const int odd_base = FMT == kFmtQ6K ? (slot_row >> 6) * ((p.k / 256 * kQ6KBlockBytes) & 15) : 0;
+    unsigned char* const a_row = a_tiles + (trow >> 3) * kSbo + (trow & 7) * 16 + half * 4 * kLbo;
+    // This thread's slabs are s = group BATCH + {0 .. BATCH - 1} + multiples of kRingGroups BATCH; buf[u], parity[u]: the
+    // buffer of the u-th of them and the parity of its last release (no divisions: they cost a slab's whole budget).  A
+    // parity wait cannot be a phase ahead: a group's slab before s is at most kRingGroups BATCH - 1 <= a_bufs back.
+    int buf[BATCH];
+    uint32_t wrapped[BATCH];  // how often the buffer has been filled before
+#pragma unroll
+    for (int u = 0; u < BATCH; ++u) buf[u] = (group * BATCH + u) % p.a_bufs, wrapped[u] = (group * BATCH + u) / p.a_bufs;
+    const int nstages = (nslabs + kPer - 1) / kPer;
+    int slot = 0, rem = (2 * (s_off / kPer) + odd_base) & 15, s = group * BATCH;
+    uint32_t rparity = 0;
+    const unsigned char* stage = ring;
+    for (int st = 0; st < nstages && !failed; ++st) {
+      if (!mbar_wait(&raw_full[slot], rparity, &g_umma_timeouts)) {
+        failed = true;
+        break;
+      }
+#pragma unroll
+      for (int si0 = 0; si0 < kPer; si0 += kRingGroups * BATCH) {
+        const int si = si0 + group * BATCH;
+        uint4 piece[BATCH][4];
+#pragma unroll
+        for (int u = 0; u < BATCH; ++u) {
+#pragma unroll
+          for (int kc = 0; kc < 4; ++kc) piece[u][kc] = make_uint4(0u, 0u, 0u, 0u);
+          if (have_row) {
+            if constexpr (FMT == kFmtQ6K) {
+              convert_q6k_stage(stage + slot_row * kQ6KPitch, rem, si + u, half, piece[u]);
+            } else {
+              RawHalf rr;
+              read_raw<FMT>(stage, trow, si + u, half, rr);
+              convert<FMT>(p, wrow, si + u, half, rr, piece[u]);
+            }
+          }
+        }
+        if (si0 + kRingGroups * BATCH >= kPer) {  // this warp is done with the stage
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&raw_empty[slot]);
+        }
+#pragma unroll
+        for (int u = 0; u < BATCH; ++u) {
+          if (s + u < nslabs) {
+            if (wrapped[u] > 0 && !mbar_wait(&empty[buf[u]], (wrapped[u] - 1) & 1, &g_umma_timeouts)) failed = true;
+#pragma unroll
+            for (int kc = 0; kc < 4; ++kc) *reinterpret_cast<uint4*>(a_row + buf[u] * kASlabBytes + kc * kLbo) = piece[u][kc];
+          }
+        }
+        fence_async_proxy();
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < BATCH; ++u) {
+          if (lane == 0 && s + u < nslabs) mbar_arrive(&full[buf[u]]);
+          buf[u] += kRingGroups * BATCH;
+          while (buf[u] >= p.a_bufs) buf[u] -= p.a_bufs, ++wrapped[u];
+        }
+        s += kRingGroups * BATCH;
+      }
+      rem = (rem + 2) & 15;
+      stage += R::kStagePitch;
+      if (++slot == p.raw_stages) slot = 0, rparity ^= 1, stage = ring;
+    }
+  } else if (warp < kRingTmaWarp) {
+    const int g = warp - kRingProducerWarps;
+    if (lane == 0 && g < issuers) {
+      // ---------------- MMA issuers -----------------------------------------
+      // Taking slabs in turn, issuer g has slabs g, g + issuers, ...; a_bufs and b_bufs are multiples of the issuers, so
+      // that a buffer always comes to the same issuer and its parity waits are never a phase ahead.  The descriptors
+      // are made once and stepped by adding to their address field.
+      const int step = by_columns ? 1 : issuers, first = by_columns ? 0 : g;
+      const int columns = !by_columns ? n_cols : g == 0 ? min(n_cols, 256) : n_cols - 256;  // (a short last chunk: none)
+      const uint32_t idesc = instr_desc(static_cast<uint32_t>(columns));
+      const uint64_t a_first = smem_desc(smem_u32(a_tiles + first * kASlabBytes));
+      const uint64_t b_first = smem_desc(smem_u32(b_tiles + first * b_slab_bytes)) + (by_columns ? g * ((256 / 8) * kSbo / 16) : 0);
+      constexpr uint64_t kKStep = 2 * kLbo / 16;
+      const uint64_t a_step = static_cast<uint64_t>(step) * (kASlabBytes / 16), b_step = static_cast<uint64_t>(step) * (b_slab_bytes / 16);
+      const uint32_t acc = tmem_base + g * acc_cols;
+      uint64_t a_desc = a_first, b_desc = b_first;
+      int buf = first, bbuf = first;
+      uint32_t parity = 0, bparity = 0, accumulate = 0;
+      for (int s = first; s < nslabs; s += step) {
+        if (!mbar_wait(&b_full[bbuf], bparity, &g_umma_timeouts) || !mbar_wait(&full[buf], parity, &g_umma_timeouts)) {
+          failed = true;
+          break;
+        }
+        tcgen05_fence_after();
+#pragma unroll
+        for (int kk = 0; kk < kSlab / 16 && columns > 0; ++kk) {
+          umma_f16(acc, a_desc + kk * kKStep, b_desc + kk * kKStep, idesc, accumulate);
+          accumulate = 1;
+        }
+        umma_commit(&empty[buf]);  // the slab buffers are free once these MMAs have read them
+        umma_commit(&b_empty[bbuf]);
+        a_desc += a_step, b_desc += b_step;
+        if ((buf += step) >= p.a_bufs) buf = first, parity ^= 1, a_desc = a_first;
+        if ((bbuf += step) >= p.b_bufs) bbuf = first, bparity ^= 1, b_desc = b_first;
+      }
+      umma_commit(done);
+    }
+  } else if (warp == kRingTmaWarp) {
+    if (lane == 0) {
+      // ---------------- TMA issuer: raw weight stages -------------------------
+      const int nstages = (nslabs + kPer - 1) / kPer;
+      int slot = 0;
+      uint32_t parity = 1;  // of the release before the stage's use; the first round has none
+      for (int st = 0; st < nstages; ++st) {
+        if (st >= p.raw_stages && !mbar_wait(&raw_empty[slot], parity, &g_umma_timeouts)) break;
+        load_raw_stage<FMT>(wmap, smap, ring + slot * R::kStagePitch, p.k, row0, s_off / kPer + st, &raw_full[slot]);
+        if (++slot == p.raw_stages) slot = 0, parity ^= 1;
+      }
+    }
+  } else if (lane == 0) {
+    // ---------------- activation copy: one bulk copy per slab ----------------
+    const unsigned char* src = p.bpre + (static_cast<size_t>(blockIdx.y) * total_slabs + s_off) * kBSlabPitch;
+    int buf = 0;
+    uint32_t parity = 1;
+    for (int s = 0; s < nslabs; ++s) {
+      if (s >= p.b_bufs && !mbar_wait(&b_empty[buf], parity, &g_umma_timeouts)) break;
+      mbar_expect_tx(&b_full[buf], static_cast<uint32_t>(b_slab_bytes));
+      bulk_load(b_tiles + buf * b_slab_bytes, src + static_cast<size_t>(s) * kBSlabPitch,
+                static_cast<uint32_t>(b_slab_bytes), &b_full[buf]);
+      if (++buf == p.b_bufs) buf = 0, parity ^= 1;
+    }
+  }
+
+  // ---------------- epilogue: TMEM -> registers -> C ------------------------
+  // a warp reads the lanes of its quadrant; the warps of a quadrant share its columns, eight at a time
+  if (warp < kRingProducerWarps) {
+    const int quad = warp & 3, part = warp >> 2;
+    const bool ok = __all_sync(0xFFFFFFFFu, !failed && mbar_wait(done, 0, &g_umma_timeouts));
+    tcgen05_fence_after();
+    if (ok) {
+      const int out_row = row0 + quad * 32 + lane;
+      float* const cz = p.c + (gridDim.z > 1 ? static_cast<size_t>(blockIdx.z) * p.m * p.n : 0);  // this k range's region
+      const float out_scale = (FMT == kFmtFp8 && out_row < p.n) ? __ldg(p.scale + out_row) : 1.0f;
+      const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
+      const int columns = p.one_term ? n_cols : tc.tok_pad;  // one term: column c is token c of the chunk
+      for (int c0 = part * 8; c0 < columns; c0 += kRingProducerWarps / 4 * 8) {
+        float v[8];
+        // by columns the second accumulator is simply column 256 and on; taking slabs in turn they are added in order
+        tmem_ld8(lane_addr + c0, v);
+        for (int g = by_columns ? issuers : 1; g < issuers; ++g) {
+          float more[8];
+          tmem_ld8(lane_addr + g * acc_cols + c0, more);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[j] += more[j];
+        }
+        if (!p.one_term) {
+          float lo[8] = {};
+          for (int g = 0; g < issuers; ++g) {
+            float more[8];
+            tmem_ld8(lane_addr + g * acc_cols + tc.tok_pad + c0, more);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) lo[j] += more[j];
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[j] += lo[j];
+        }
+        if (out_row < p.n) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (c0 + j < tc.tokens) cz[static_cast<size_t>(tc.tok0 + c0 + j) * p.n + out_row] = v[j] * out_scale;
+        }
+      }
+    }
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  if (warp == kRingProducerWarps) tmem_dealloc(tmem_base, tmem_cols);
+}
+
 // ---- tensor maps of the raw ring (cached per weight tensor) ---------------------
 struct RingMaps {
   CUtensorMap weights, scales;
@@ -677,6 +978,14 @@ int ring_maps(int fmt, const void* w, uint64_t n, uint64_t k, RingMaps* out) {
     const uint32_t box[3] = {18, 1, kTileM};
     rc = encode_tensor_map(&maps.weights, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, w, dims, strides, box);
     maps.scales = maps.weights;
+  } else if (fmt == kFmtQ6K) {
+    const uint64_t row_bytes = k / 256 * kQ6KBlockBytes, odd = row_bytes & 15;  // 0 or 8
+    const auto* base = static_cast<const unsigned char*>(w);
+    const uint64_t strides[1] = {2 * row_bytes};
+    const uint32_t box[2] = {kQ6KPitch / 8, kTileM / 2};
+    const uint64_t even_dims[2] = {row_bytes / 8, (n + 1) / 2}, odd_dims[2] = {(row_bytes + odd) / 8, n / 2};
+    rc = encode_tensor_map(&maps.weights, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, base, even_dims, strides, box);
+    if (rc == kOk) rc = encode_tensor_map(&maps.scales, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, base + row_bytes - odd, odd_dims, strides, box);
   } else {
     const uint64_t row_bytes = fmt == kFmtMxFp4 ? k / 2 : k;
     const uint64_t dims[3] = {128, n, row_bytes / 128};
@@ -756,11 +1065,11 @@ int launch_umma_impl(UmmaParams p, const RingMaps& maps, cudaStream_t st, bool a
   const int two_term_rows = (FMT == kFmtQ4K || FMT == kFmtQ6K) ? kMaxTokens : 2 * kMaxTokens;
   const bool narrow = p.m > two_term_rows && std::getenv("TSR_TILE_TWO_TERMS") == nullptr;
   // Tokens per CTA: the widest stage is the cheapest per token, but only while the grid still covers the SMs:
-  // relative time of one CTA per stage (measured on Q4_K 17408 x 5120: 491 / 787 / 1018 TFLOP/s at 128 / 256 /
-  // 512 tokens per CTA) times the waves its grid needs.  5120 weight rows are 40 row tiles: 512 tokens in
+  // relative time of one CTA per stage (measured on Q4_K 17408 x 5120: 41 / 63 / 84 us for 128 / 256 / 512 columns of
+  // operand B per CTA) times the waves its grid needs.  5120 weight rows are 40 row tiles: 512 tokens in
   // one chunk would leave 108 SMs idle, two chunks of 256 finish in two thirds of the time.
   // ... and where the grid of the widest stage still leaves half of the SMs idle (5120 weight rows: 40 row
-  // tiles), k is cut among up to four CTAs per tile, whose partial sums gemm_vec_reduce adds.
+  // tiles), k is cut among several CTAs per tile, whose partial sums gemm_vec_reduce adds.
   int widest = !narrow ? 0 : (p.m > 2 * kMaxTokens && allow_scratch && std::getenv("TSR_TILE_128") == nullptr)
                                  ? ((p.m > 4 * kMaxTokens && std::getenv("TSR_TILE_256") == nullptr) ? 3 : 2) : 1;
   constexpr int kPerStage = RING ? RingFmt<FMT>::kSlabsPerStage : 4;
@@ -773,18 +1082,19 @@ int launch_umma_impl(UmmaParams p, const RingMaps& maps, cudaStream_t st, bool a
       cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
       return v > 0 ? v : 148;
     }();
-    const double unit[4] = {0.5, 0.509, 0.635, 0.982};
+    const double unit[4] = {0.48, 0.49, 0.74, 0.98};
     const long tiles = (p.n + kTileM - 1) / kTileM;
-    const int max_split = (allow_scratch && std::getenv("TSR_TILE_NO_KSPLIT") == nullptr) ? 4 : 1;
+    const int max_split = (allow_scratch && std::getenv("TSR_TILE_NO_KSPLIT") == nullptr) ? 8 : 1;
+    const double split_cost = 0.06 * 5120.0 / p.k;  // 5 us of 84 at k = 5120
     double best = 0.0;
     int pick = widest;
     for (int mode = widest; mode >= (widest >= 2 ? 1 : widest); --mode) {
       const long per = static_cast<long>(kMaxTokens) << mode;
       const long ctas = tiles * ((p.m + per - 1) / per);
       for (int sp = 1; sp <= max_split; ++sp) {
-        if (sp > 1 && (ctas * sp > sms || stages_total / sp < 16)) break;  // one wave, and enough k left per CTA (4096)
+        if (sp > 1 && (ctas * sp > sms || stages_total * kPerStage / sp < 20)) break;  // one wave, and enough k left per CTA (1280)
         // a split costs the fill and drain of every CTA's pipeline again and the sum of the partial regions
-        const double cost = static_cast<double>((ctas * sp + sms - 1) / sms) * (unit[mode] / sp + (sp > 1 ? 0.06 : 0.0));
+        const double cost = static_cast<double>((ctas * sp + sms - 1) / sms) * (unit[mode] / sp + (sp > 1 ? split_cost : 0.0));
         if ((mode == widest && sp == 1) || cost < best * 0.9) best = cost, pick = mode, ksplit = sp;  // must win clearly
       }
     }
@@ -792,16 +1102,33 @@ int launch_umma_impl(UmmaParams p, const RingMaps& maps, cudaStream_t st, bool a
   }
   p.one_term = widest;
   const int nslabs = p.k / kSlab;
-  const size_t ring = RING ? static_cast<size_t>(kRawStages) * RingFmt<FMT>::kStagePitch : 0;
+  // Shared memory of a CTA with the given buffers.  The weight slabs have more buffers than the activation slabs where
+  // they fit: the producers' latency (raw bytes, arithmetic, stores, fence) is longer than the MMAs of a slab, and with
+  // one common pair of buffers it showed on every slab.
+  auto smem_of = [&](int a_bufs, int b_bufs, int raw_stages, int tok_pad) -> size_t {
+    return 1024 + (RING ? static_cast<size_t>(raw_stages) * RingFmt<FMT>::kStagePitch : 0) + a_bufs * kASlabBytes +
+           b_bufs * static_cast<size_t>(2 * tok_pad) * kSlab * 2 + 512;
+  };
   dim3 grid;
   size_t smem = 0;
   for (;;) {
     const int tok_pad = token_chunk(p.m, 0, p.one_term).tok_pad;  // the first chunk is the largest
     const int per_cta = kMaxTokens << p.one_term;
-    smem = 1024 + ring + kBufs * kASlabBytes + kBufs * static_cast<size_t>(2 * tok_pad) * kSlab * 2 + 256;
     grid = dim3(static_cast<unsigned>((p.n + kTileM - 1) / kTileM), static_cast<unsigned>((p.m + per_cta - 1) / per_cta));
     // activations -> operand layout once per launch, when scratch is to be had
     p.bpre = allow_scratch ? activation_scratch(st, static_cast<size_t>(grid.y) * nslabs * kBSlabPitch) : nullptr;
+    // Buffers: the ring kernel's issuers that take slabs in turn want multiples of their number (two rounds of the
+    // producers' groups are four weight slabs as well), 512 columns three weight slabs where they fit; then raw stages.
+    const int n_cols = 2 * tok_pad;
+    p.by_columns = n_cols > 256 ? 1 : 0;
+    p.issuers = n_cols > 128 ? 2 : kMaxIssuers;
+    const bool turns = RING && p.bpre != nullptr && !p.by_columns;
+    p.b_bufs = turns ? p.issuers : kBufs;
+    p.a_bufs = turns ? 4 : kBufs;
+    p.raw_stages = kBufs;
+    if (RING && p.bpre != nullptr && !turns && smem_of(3, p.b_bufs, p.raw_stages, tok_pad) <= 227 * 1024) p.a_bufs = 3;
+    while (RING && p.raw_stages < kMaxRaw && smem_of(p.a_bufs, p.b_bufs, p.raw_stages + 1, tok_pad) <= 227 * 1024) ++p.raw_stages;
+    smem = smem_of(p.a_bufs, p.b_bufs, p.raw_stages, tok_pad);
     if (p.one_term >= 2 && (p.bpre == nullptr || smem > 227 * 1024)) {  // no scratch, or the ring leaves no room
       --p.one_term;
       continue;
@@ -810,7 +1137,7 @@ int launch_umma_impl(UmmaParams p, const RingMaps& maps, cudaStream_t st, bool a
   }
   if (int rc = allow_dynamic_smem(reinterpret_cast<const void*>(&gemm_umma_kernel<FMT, RING>), 227 * 1024)) return rc;
   if (p.bpre != nullptr) {
-    convert_activations_kernel<<<dim3(nslabs, grid.y), 256, 0, st>>>(p.a, const_cast<unsigned char*>(p.bpre), p.m, p.k, p.one_term);
+    convert_activations_kernel<<<dim3(nslabs, grid.y, p.one_term == 3 ? 8 : p.one_term == 2 ? 4 : 2), 256, 0, st>>>(p.a, const_cast<unsigned char*>(p.bpre), p.m, p.k, p.one_term);
     if (int rc = check_launch()) return rc;
   }
   float* const out = p.c;
@@ -822,7 +1149,17 @@ int launch_umma_impl(UmmaParams p, const RingMaps& maps, cudaStream_t st, bool a
     if (part == nullptr) ksplit = 1;
     else p.c = part, grid.z = static_cast<unsigned>(ksplit);
   }
-  gemm_umma_kernel<FMT, RING><<<grid, kUmmaThreads, smem, st>>>(maps.weights, maps.scales, p);
+  bool launched = false;
+  if constexpr (RING) {
+    if (p.bpre != nullptr) {
+      // two slabs a round while a group never waits for a buffer that its own unpublished slab holds up
+      auto kernel = p.a_bufs >= 3 ? gemm_umma_ring_kernel<FMT, 2> : gemm_umma_ring_kernel<FMT, 1>;
+      if (int rc = allow_dynamic_smem(reinterpret_cast<const void*>(kernel), 227 * 1024)) return rc;
+      kernel<<<grid, kRingThreads, smem, st>>>(maps.weights, maps.scales, p);
+      launched = true;
+    }
+  }
+  if (!launched) gemm_umma_kernel<FMT, RING><<<grid, kUmmaThreads, smem, st>>>(maps.weights, maps.scales, p);
   if (int rc = check_launch()) return rc;
   if (ksplit > 1) return tsr_gemm_vec_reduce(p.c, out, static_cast<uint64_t>(p.m) * p.n, static_cast<uint64_t>(ksplit), st);
   return kOk;
@@ -832,12 +1169,12 @@ template <int FMT>
 int launch_umma(const UmmaParams& p, cudaStream_t st, bool allow_scratch) {
   // the ring wants whole segments (and 16-byte scale rows for MXFP4) and 16-byte aligned weights
   const bool aligned = (reinterpret_cast<uintptr_t>(p.w) & 15u) == 0;
-  const bool ring = aligned && (FMT == kFmtQ4K || (FMT == kFmtFp8 && p.k % 128 == 0) ||
-                                (FMT == kFmtMxFp4 && p.k % 512 == 0));
+  const bool ring = aligned && (FMT == kFmtQ4K || (FMT == kFmtQ6K && p.k % 1024 == 0 && p.n >= 2) ||
+                                (FMT == kFmtFp8 && p.k % 128 == 0) || (FMT == kFmtMxFp4 && p.k % 512 == 0));
   RingMaps maps{};
-  if (ring && FMT != kFmtQ6K) {
+  if (ring) {
     if (int rc = ring_maps(FMT, p.w, static_cast<uint64_t>(p.n), static_cast<uint64_t>(p.k), &maps)) return rc;
-    return launch_umma_impl<FMT, FMT != kFmtQ6K>(p, maps, st, allow_scratch);
+    return launch_umma_impl<FMT, true>(p, maps, st, allow_scratch);
   }
   return launch_umma_impl<FMT, false>(p, maps, st, allow_scratch);
 }

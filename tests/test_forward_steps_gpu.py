@@ -272,3 +272,16 @@ def test_head_sized_rows(backend, oracle, rows, cols):
     y = backend.download(yb, np.float32, rows * cols + 7)
     assert close(y[3:-4], oracle.rmsnorm_gated(x, w, gate, 1e-6).reshape(-1), 2e-6)
     assert np.all(y[:3] == np.float32(-3e9)) and np.all(y[-4:] == np.float32(-3e9))
+
+
+@pytest.mark.parametrize("n", [1 << 16, (1 << 16) + 4, (1 << 16) + 1, 65532])
+def test_wide_elementwise_steps(backend, oracle, n):
+    """silu_mul and add on both sides of the four-wide kernels' limit, and in place."""
+    g = np.random.default_rng(n)
+    x, y = g.standard_normal(n).astype(np.float32), g.standard_normal(n).astype(np.float32)
+    out = backend.AllocateBuffer(n * 4)
+    run(backend, "silu_mul", [backend.upload(x), backend.upload(y), out], [n])
+    assert close(backend.download(out, np.float32, n), oracle.silu_mul(x, y), 2e-6)
+    xb = backend.upload(x)
+    run(backend, "add", [xb, backend.upload(y), xb], [n])
+    assert np.array_equal(backend.download(xb, np.float32, n), x + y)

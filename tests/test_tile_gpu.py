@@ -123,3 +123,34 @@ def test_prefill_sized_batches(backend, oracle, m):
         # both operands of every product are rounded to binary16 here (as in the reference's own tile): single
         # outputs near zero reach 2.1e-3 of the vector's rms, measured; the max-relative form above is at 4e-4
         assert per_element_ok(got, ref, tol=3e-3)
+
+
+@pytest.mark.parametrize("m,n,k", [(40, 128, 1024), (70, 131, 1024), (33, 129, 2048), (520, 257, 3072), (260, 64, 1024),
+                                   (65, 200, 768), (600, 130, 1024)])
+def test_q6k_blocks_from_the_ring(backend, oracle, m, n, k):
+    """The raw ring of the Q6_K tile (even and odd rows as two tensors): odd row counts, k/256 with an 8-byte and a
+    16-byte aligned odd row, one and two activation terms, a last chunk narrower than the first, and a k the ring
+    leaves to the direct loads.  Weights and activations are rounded to binary16: 1e-3 as for the other formats."""
+    a = synth.activations(m, k, seed=60)
+    w = synth.q6k_weights(n, k, seed=61)
+    out = padded_output(backend, m * n)
+    launch(backend, "gemm_q6k_batched", [backend.upload(a), backend.upload(w), out], [m, n, k])
+    got, tail = read_padded(backend, out, m * n)
+    assert np.all(tail == CANARY)
+    ref = oracle.gemm_q6k(a, w, m, n, k)
+    assert rel_err(got.reshape(m, n), ref) < 1e-3
+    assert per_element_ok(got.reshape(m, n), ref, tol=3e-3)
+
+
+@pytest.mark.parametrize("m,n,k", [(30, 128, 128), (30, 130, 384), (64, 128, 256), (100, 100, 1280), (300, 128, 128), (128, 1000, 4096)])
+def test_few_slabs_and_issuers(backend, oracle, m, n, k):
+    """FP8 batches on the ring kernel with fewer slabs than issuers, slabs that are no multiple of them, a stage half
+    beyond k, and a k cut among CTAs.  Up to 128 rows two binary16 terms per activation: fp32-like results."""
+    a = synth.activations(m, k, seed=70)
+    w, s = synth.fp8_weights(n, k, seed=71)
+    out = padded_output(backend, m * n)
+    launch(backend, "gemm_fp8", [backend.upload(a), backend.upload(w), backend.upload(s), out], [m, n, k])
+    got, tail = read_padded(backend, out, m * n)
+    assert np.all(tail == CANARY)
+    ref = oracle.gemm_fp8(a, w, s, m, n, k)
+    assert rel_err(got.reshape(m, n), ref) < (2e-5 if m <= 128 else 1e-3)
