@@ -48,6 +48,56 @@ quantize_fp8_kernel(float* __restrict__ data, const float* __restrict__ in,
   }
 }
 
+// The code float_to_e4m3_ref gives a value in [-448, 448] (or a NaN), from the hardware's conversion: both round to
+// nearest even, but the reference clamps a subnormal's mantissa at 7 where rounding would carry into the smallest normal
+// value, and keeps a NaN's sign.
+__device__ __forceinline__ uint32_t e4m3_code(float q) {
+  const uint32_t bits = __float_as_uint(q), sign = (bits >> 31) << 7;
+  const float mag = fabsf(q);
+  uint32_t code = __nv_cvt_float_to_fp8(q, __NV_SATFINITE, __NV_E4M3);
+  if (mag >= 7.5f / 512.0f && mag < 8.0f / 512.0f) code = sign | 7u;
+  return q == q ? code : (sign | 0x7Fu);
+}
+
+// The codes of a batch (quantize_fp8_pack) with several CTAs per row: each finds the row's maximum by itself (the row is
+// a few tens of KB, served from L2 after the first) and codes its share, four columns a thread.  One CTA a row left 16
+// verify rows on 16 SMs, with frexp and a 64-bit rounding an element: 16 rows of 5120 / 17408 took 7.3 / 17.6 us, here
+// 3.7 / 5.2.
+constexpr int kPackThreads = 512;
+__global__ void __launch_bounds__(kPackThreads)
+quantize_fp8_pack_kernel(const float4* __restrict__ in, uint32_t* __restrict__ codes, float* __restrict__ scale, int cols4) {
+  __shared__ float red[kPackThreads / 32];
+  const size_t base = static_cast<size_t>(blockIdx.x) * cols4;
+  float amax = 0.0f;
+#pragma unroll 4
+  for (int c = threadIdx.x; c < cols4; c += kPackThreads) {
+    const float4 x = __ldg(in + base + c);
+    amax = fmaxf(amax, fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))));  // fmaxf drops NaN like std::max
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
+  __syncthreads();
+  amax = red[0];
+#pragma unroll
+  for (int w = 1; w < kPackThreads / 32; ++w) amax = fmaxf(amax, red[w]);
+  const float s = fmaxf(__fdiv_rn(amax, 448.0f), 1.0f / (448.0f * 512.0f));
+  if (blockIdx.y == 0 && threadIdx.x == 0) scale[blockIdx.x] = s;
+  const int share = (cols4 + gridDim.y - 1) / gridDim.y, c0 = blockIdx.y * share, c1 = min(cols4, c0 + share);
+  for (int c = c0 + threadIdx.x; c < c1; c += kPackThreads) {
+    const float4 x = __ldg(in + base + c);
+    const float v[4] = {x.x, x.y, x.z, x.w};
+    uint32_t w = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float q = __fdiv_rn(v[i], s);
+      q = q < -448.0f ? -448.0f : (448.0f < q ? 448.0f : q);  // std::clamp; NaN passes through
+      w |= e4m3_code(q) << (8 * i);
+    }
+    codes[base + c] = w;
+  }
+}
+
 // gemm_vec_reduce.comp:20-32: ordered sum of the split regions.
 __global__ void vec_reduce_kernel(const float* __restrict__ part, float* __restrict__ c,
                                   size_t total, int split) {
@@ -243,6 +293,14 @@ int tsr_quantize_fp8_pack(const float* in, void* out, float* scale, uint64_t row
                           void* stream) {
   if (!in || !out || !scale || rows == 0 || cols == 0 || cols % 4 != 0 || cols > 0x7FFFFFFFull)
     return kInvalidArgument;
+  if (((reinterpret_cast<uintptr_t>(in) & 15u) | (reinterpret_cast<uintptr_t>(out) & 3u)) == 0 && rows <= 0x7FFFFFFFull) {
+    // CTAs per row: up to two per SM over all rows, at least 1024 columns each
+    const uint64_t most = (cols + 1023) / 1024, want = (296 + rows - 1) / rows;
+    const unsigned parts = static_cast<unsigned>(want < most ? want : most);
+    quantize_fp8_pack_kernel<<<dim3(static_cast<unsigned>(rows), parts), kPackThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+        reinterpret_cast<const float4*>(in), static_cast<uint32_t*>(out), scale, static_cast<int>(cols / 4));
+    return check_launch();
+  }
   quantize_fp8_kernel<true><<<static_cast<unsigned>(rows), 1024, 0,
                               static_cast<cudaStream_t>(stream)>>>(
       nullptr, in, static_cast<uint8_t*>(out), scale, static_cast<int>(cols));

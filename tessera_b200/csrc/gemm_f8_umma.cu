@@ -27,8 +27,8 @@
 //
 // Per CTA: 128 weight rows, one range of k; warp 0 issues the TMA copies of a
 // four-stage ring (two 128-byte k segments of weights and of activation terms
-// per stage), warp 1 issues eight K = 32 MMAs per stage into TMEM and commits
-// them to the stage's empty barrier, warps 2-5 read the accumulator with
+// per stage), warps 1 and 2 issue four K = 32 MMAs each per stage into TMEM and commit
+// them to the stage's empty barrier, warps 3-6 read the accumulators with
 // tcgen05.ld and store C (or this CTA's partial sums when k is split over
 // CTAs; the regions are then added in order by the reduce kernel).  Every
 // wait is bounded and TMEM is released on every path.
@@ -57,7 +57,9 @@ constexpr int kSegs = 2;        // segments per stage
 constexpr int kMaxStages = 4;
 constexpr int kTerms = 3;
 constexpr int kMaxCols = 64;  // B columns (activation rows x terms, padded to 16)
-constexpr int kThreads = 6 * 32;
+constexpr int kIssuers = kSegs;  // MMA issuers: one per segment of a stage
+constexpr int kEpilogueWarp = 1 + kIssuers;
+constexpr int kThreads = (kEpilogueWarp + 4) * 32;
 constexpr int kWeightStage = kSegs * kTileM * kSegBytes;  // 32 KiB
 
 enum : int { kFp8 = 0, kMxFp4 = 1 };
@@ -121,6 +123,17 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
   for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// Adds the other issuers' accumulators to eight columns of the first one's.
+__device__ __forceinline__ void add_columns(uint32_t lane_addr, int col, int ncols, float* v) {
+#pragma unroll
+  for (int g = 1; g < kIssuers; ++g) {
+    float more[8];
+    tmem_ld8(lane_addr + g * ncols + col, more);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] += more[i];
+  }
 }
 
 // Shared-memory matrix descriptor of a K-major tile whose rows are 128 bytes, stored with
@@ -249,21 +262,21 @@ gemm_f8_umma_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
   const int row0 = blockIdx.x * kTileM;
   const int stage0 = blockIdx.y * p.stages_per_cta;
   const int nstages = min(p.stages_per_cta, p.total_stages - stage0);
-  // tensor memory: the accumulator, then (MXFP4) four scale-factor columns per segment of
-  // every ring stage and four for the B side
-  const uint32_t sfa_col = static_cast<uint32_t>(p.ncols), sfb_col = sfa_col + kMaxStages * kSegs * 4;
+  // tensor memory: an accumulator per issuer, then (MXFP4) four scale-factor columns per segment of
+  // every ring stage and four per issuer for the B side
+  const uint32_t sfa_col = static_cast<uint32_t>(kIssuers * p.ncols), sfb_col = sfa_col + kMaxStages * kSegs * 4;
   uint32_t tmem_cols = 32;
-  while (tmem_cols < (FMT == kMxFp4 ? sfb_col + 4 : static_cast<uint32_t>(p.ncols))) tmem_cols <<= 1;
+  while (tmem_cols < (FMT == kMxFp4 ? sfb_col + 4 * kIssuers : sfa_col)) tmem_cols <<= 1;
 
   if (tid == 0) {
     tma_prefetch_descriptor(&wmap);
     tma_prefetch_descriptor(&bmap);
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&full[s], 1);
-      mbar_init(&empty[s], 1);
+      mbar_init(&empty[s], kIssuers);
       mbar_init(&sf_full[s], 4);  // one arrival per epilogue warp
     }
-    mbar_init(done, 1);
+    mbar_init(done, kIssuers);
     mbar_fence_init();
   }
   if (warp == 1) tmem_alloc(tmem_slot, tmem_cols);
@@ -300,43 +313,49 @@ gemm_f8_umma_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         tma_load_3d(b_tiles + slot * b_stage, &bmap, 0, 0, kSegs * (stage0 + s), &full[slot]);
       }
     }
-  } else if (warp == 1) {
+  } else if (warp < kEpilogueWarp) {
     if (lane == 0) {
-      // ---------------- MMA issuer ------------------------------------------------
+      // ---------------- MMA issuers ------------------------------------------------
+      // A stage costs its issuing thread more than the tensor pipe (two waits of about 230 cycles, 120 a MMA, the
+      // commit), so each segment of a stage has an issuer and an accumulator of its own; every issuer waits for every
+      // stage, in order.
+      const int seg = warp - 1;
+      const uint32_t acc = tmem_base + static_cast<uint32_t>(seg * p.ncols), sfb = tmem_base + sfb_col + 4 * seg;
       const uint32_t idesc = instr_desc(static_cast<uint32_t>(p.ncols));
+      const uint64_t a_first = smem_desc_sw128(smem_u32(w_tiles + seg * kTileM * kSegBytes));
+      const uint64_t b_first = smem_desc_sw128(smem_u32(b_tiles + seg * p.ncols * kSegBytes));
+      const uint64_t b_step = static_cast<uint64_t>(b_stage / 16);
+      uint64_t adesc = a_first, bdesc = b_first;
+      uint32_t parity = 0, accumulate = 0;
+      int slot = 0;
       bool ok = true;
-      for (int s = 0; s < nstages; ++s) {
-        const int slot = s % kStages, round = s / kStages;
-        if (!mbar_wait(&full[slot], round & 1, &g_f8_timeouts) ||
-            (FMT == kMxFp4 && !mbar_wait(&sf_full[slot], round & 1, &g_f8_timeouts))) {
+      if (FMT == kMxFp4 && nstages > 0) {
+        // the ones of the B side are in shared memory when the first stage's scale factors are
+        ok = mbar_wait(&sf_full[0], 0, &g_f8_timeouts);
+        tcgen05_fence_after();
+        if (ok) tmem_cp_32x128b_x4(sfb, smem_desc_sf(smem_u32(sf_ones)));
+      }
+      for (int s = 0; s < nstages && ok; ++s) {
+        if (!mbar_wait(&full[slot], parity, &g_f8_timeouts) ||
+            (FMT == kMxFp4 && !mbar_wait(&sf_full[slot], parity, &g_f8_timeouts))) {
           ok = false;
           break;
         }
         tcgen05_fence_after();
-        const uint32_t a_addr = smem_u32(w_tiles + slot * kWeightStage), b_addr = smem_u32(b_tiles + slot * b_stage);
-        if (FMT == kMxFp4) {
-          if (s == 0) tmem_cp_32x128b_x4(tmem_base + sfb_col, smem_desc_sf(smem_u32(sf_ones)));
+        const uint32_t sfa = tmem_base + sfa_col + (slot * kSegs + seg) * 4;
+        if (FMT == kMxFp4) tmem_cp_32x128b_x4(sfa, smem_desc_sf(smem_u32(sf_stage + (slot * kSegs + seg) * 512)));
 #pragma unroll
-          for (int seg = 0; seg < kSegs; ++seg)
-            tmem_cp_32x128b_x4(tmem_base + sfa_col + (slot * kSegs + seg) * 4,
-                               smem_desc_sf(smem_u32(sf_stage + (slot * kSegs + seg) * 512)));
-        }
-#pragma unroll
-        for (int seg = 0; seg < kSegs; ++seg) {
-#pragma unroll
-          for (int kk = 0; kk < kSegBytes / 32; ++kk) {
-            const uint64_t adesc = smem_desc_sw128(a_addr + seg * kTileM * kSegBytes + kk * 32);
-            const uint64_t bdesc = smem_desc_sw128(b_addr + seg * p.ncols * kSegBytes + kk * 32);
-            const uint32_t acc = (s > 0 || seg > 0 || kk > 0) ? 1u : 0u;
-            if (FMT == kMxFp4) {
-              umma_mxf8f6f4(tmem_base, adesc, bdesc, instr_desc_mx(static_cast<uint32_t>(p.ncols), kk),
-                            tmem_base + sfa_col + (slot * kSegs + seg) * 4, tmem_base + sfb_col, acc);
-            } else {
-              umma_f8(tmem_base, adesc, bdesc, idesc, acc);
-            }
+        for (int kk = 0; kk < kSegBytes / 32; ++kk) {
+          if (FMT == kMxFp4) {
+            umma_mxf8f6f4(acc, adesc + kk * 2, bdesc + kk * 2, instr_desc_mx(static_cast<uint32_t>(p.ncols), kk), sfa, sfb, accumulate);
+          } else {
+            umma_f8(acc, adesc + kk * 2, bdesc + kk * 2, idesc, accumulate);
           }
+          accumulate = 1;
         }
-        umma_commit(&empty[slot]);  // the stage is free once these MMAs have read it
+        umma_commit(&empty[slot]);  // the stage is free once both segments' MMAs have read it
+        adesc += kWeightStage / 16, bdesc += b_step;
+        if (++slot == kStages) slot = 0, parity ^= 1, adesc = a_first, bdesc = b_first;
       }
       if (ok) umma_commit(done);
     }
@@ -349,7 +368,7 @@ gemm_f8_umma_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
       // row's scale word of each segment (four E8M0 bytes, one per K block of 32) where
       // tcgen05.cp.32x128b.warpx4 wants it: row t % 32 of the 512-byte piece, word t / 32.  The
       // words come straight from the side table, a few stages ahead of their use.
-      const int et = tid - 64;  // 0..127
+      const int et = tid - kEpilogueWarp * 32;  // 0..127
       const int grow = row0 + et;
       const int sf_words = p.k / 128;  // scale words per weight row
       const uint32_t* sf_row = reinterpret_cast<const uint32_t*>(p.sf + static_cast<size_t>(grow < p.n ? grow : 0) * (p.k / 32));
@@ -396,6 +415,7 @@ gemm_f8_umma_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         for (int c0 = 0; c0 < p.ncols; c0 += 8) {
           float d[8];
           tmem_ld8(lane_addr + c0, d);
+          add_columns(lane_addr, c0, p.ncols, d);
           if (out_row < p.n) {
 #pragma unroll
             for (int j = 0; j < 8; ++j)
@@ -410,6 +430,7 @@ gemm_f8_umma_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         for (int q = 0; q < 3; ++q) {
           if (c0 + 8 * q < p.ncols) {
             tmem_ld8(lane_addr + c0 + 8 * q, d + 8 * q);
+            add_columns(lane_addr, c0 + 8 * q, p.ncols, d + 8 * q);
           } else {
 #pragma unroll
             for (int j = 0; j < 8; ++j) d[8 * q + j] = 0.0f;

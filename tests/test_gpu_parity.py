@@ -427,3 +427,23 @@ def test_copies_round_trip(backend):
     total, free = backend.MemoryInfo()
     assert total > free > 0
     assert "B200" in backend.DeviceName() or backend.DeviceName()
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 4), (3, 1028), (16, 5120), (300, 260)])
+def test_fp8_codes_around_every_rounding_boundary(backend, oracle, rows, cols):
+    """quantize_fp8_pack_rows over values that hit ties, the subnormals up to the clamp below the smallest normal value,
+    signed zeros, a NaN and an all-zero row, with one and several CTAs a row: codes and scales bit for bit."""
+    g = np.random.default_rng(rows + cols)
+    grid = np.concatenate([np.arange(0, 129, dtype=np.float64) / 1024.0, np.arange(8, 128) / 256.0 * 1.0, 2.0 ** np.arange(-12, 8),
+                           448.0 * g.random(600)])
+    x = (g.choice(grid, size=(rows, cols)) * g.choice([-1.0, 1.0], size=(rows, cols))).astype(np.float32)
+    x[:, 0] = 448.0     # the scale is one: the codes are those of the values themselves
+    if rows > 2:
+        x[1] = 0.0
+        x[2, 1:3] = [np.nan, -0.0]
+    out, sc = backend.AllocateBuffer(rows * cols), backend.AllocateBuffer(rows * 4)
+    backend.LaunchKernel(backend.LoadKernel("quantize_fp8_pack_rows"),
+                         KernelLaunch(buffers=[backend.upload(x), out, sc], scalars=[rows, cols]))
+    codes, scale = oracle.quantize_fp8_pack(x)
+    assert np.array_equal(backend.download(sc, np.float32, rows), scale)
+    assert np.array_equal(backend.download(out, np.uint8, rows * cols), codes.reshape(-1))
