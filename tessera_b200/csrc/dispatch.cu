@@ -1277,6 +1277,49 @@ size_t merged_attention_gate(tsr_context* ctx, const std::vector<PendingLaunch>&
   return *rc == kUnsupportedFeature ? 0 : 2;
 }
 
+// top_k_rows of one row, moe_gate on its values (the router of an expert layer)
+size_t merged_router(tsr_context* ctx, const std::vector<PendingLaunch>& q, size_t i, int* rc) {
+  if (!ctx->fold_elementwise || !fuse_elementwise() || i + 2 > q.size() || !is_named(q[i], "top_k_rows") || !is_named(q[i + 1], "moe_gate"))
+    return 0;
+  const PendingLaunch &tk = q[i], &mg = q[i + 1];
+  const uint64_t vocab = tk.sc[1], top_k = tk.sc[2], hidden = mg.sc[1];
+  if (tk.sc[0] != 1 || tk.sc[3] != 0 || mg.sc[0] != top_k || mg.buf[0] != tk.buf[2]) return 0;
+  // the kernel reads the gate's operands before the values are written and writes the gates after: buffers apart
+  const struct { const void* p; uint64_t bytes; } reads[3] = {{tk.buf[0], vocab * 4}, {mg.buf[1], hidden * 4}, {mg.buf[2], hidden * 4}},
+                                                  writes[4] = {{tk.buf[1], top_k * 4}, {tk.buf[2], top_k * 4}, {mg.buf[3], top_k * 4}, {mg.buf[4], 4}};
+  for (int w = 0; w < 4; ++w) {
+    for (const auto& r : reads)
+      if (overlaps(writes[w].p, writes[w].bytes, r.p, r.bytes)) return 0;
+    for (int o = 0; o < w; ++o)
+      if (overlaps(writes[w].p, writes[w].bytes, writes[o].p, writes[o].bytes)) return 0;
+  }
+  *rc = launch_router_select(fbuf(tk, 0), static_cast<uint32_t*>(const_cast<void*>(tk.buf[1])), fbuf(tk, 2), fbuf(mg, 1), fbuf(mg, 2),
+                             fbuf(mg, 3), fbuf(mg, 4), vocab, top_k, hidden, ctx->stream);
+  return *rc == kUnsupportedFeature ? 0 : 2;
+}
+
+// moe_scale_add, add of its result (the residual)
+size_t merged_scale_add(tsr_context* ctx, const std::vector<PendingLaunch>& q, size_t i, int* rc) {
+  if (!ctx->fold_elementwise || !fuse_elementwise() || i + 2 > q.size() || !is_named(q[i], "moe_scale_add") || !is_named(q[i + 1], "add"))
+    return 0;
+  const PendingLaunch &sa = q[i], &ad = q[i + 1];
+  const uint64_t n = sa.sc[0], bytes = n * 4;
+  if (ad.sc[0] != n) return 0;
+  const void* base = ad.buf[0] == sa.buf[3] ? ad.buf[1] : ad.buf[1] == sa.buf[3] ? ad.buf[0] : nullptr;
+  if (base == nullptr || overlaps(base, bytes, sa.buf[3], bytes)) return 0;
+  // element by element, so an output may be an input in place, not a shifted overlap; the factor is read by everybody
+  const void* out = ad.buf[2];
+  for (const void* o : {sa.buf[3], out}) {
+    for (const void* r : {sa.buf[0], sa.buf[1], base})
+      if (o != r && overlaps(o, bytes, r, bytes)) return 0;
+    if (overlaps(o, bytes, static_cast<const float*>(sa.buf[2]) + sa.sc[1], 4)) return 0;
+  }
+  if (overlaps(out, bytes, sa.buf[3], bytes)) return 0;
+  *rc = launch_moe_scale_add_add(fbuf(sa, 0), fbuf(sa, 1), fbuf(sa, 2), fbuf(sa, 3), static_cast<const float*>(base), fbuf(ad, 2), n,
+                                 sa.sc[1], ctx->stream);
+  return 2;
+}
+
 int issue_one(tsr_context* ctx, const PendingLaunch& op) {
   const Args a{op.buf, op.bytes, op.nbuf, op.sc, op.nsc, op.grid_y, ctx->stream, false, ctx};
   return kTable[op.kernel].fn(a);
@@ -1297,6 +1340,8 @@ int issue_queue(tsr_context* ctx, const std::vector<PendingLaunch>& q) {
       size_t merged = merged_linear_mixer_inputs(ctx, q, i, &rc);
       if (merged == 0) merged = merged_head_norm_rope(ctx, q, i, &rc);
       if (merged == 0) merged = merged_attention_gate(ctx, q, i, &rc);
+      if (merged == 0) merged = merged_router(ctx, q, i, &rc);
+      if (merged == 0) merged = merged_scale_add(ctx, q, i, &rc);
       if (merged != 0) {
         if (rc != kOk) return rc;
         i += merged;

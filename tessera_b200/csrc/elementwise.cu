@@ -235,9 +235,19 @@ __global__ void __launch_bounds__(256) add4_kernel(const float4* a, const float4
 __global__ void __launch_bounds__(1024)
 rmsnorm_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y, int cols, float eps) {
   __shared__ float red[32];
+  constexpr int kHeld = 8;  // of a thread's columns, the first eight stay in registers: their loads are in flight together
   const float* row = x + static_cast<size_t>(blockIdx.x) * cols;
+  float held[kHeld], weight[kHeld];
+#pragma unroll
+  for (int i = 0; i < kHeld; ++i) {
+    const int c = threadIdx.x + i * blockDim.x;
+    held[i] = c < cols ? row[c] : 0.0f;
+    weight[i] = c < cols ? __ldg(w + c) : 0.0f;
+  }
   float s = 0.0f;
-  for (int c = threadIdx.x; c < cols; c += blockDim.x) s = fmaf(row[c], row[c], s);
+#pragma unroll
+  for (int i = 0; i < kHeld; ++i) s = fmaf(held[i], held[i], s);
+  for (int c = threadIdx.x + kHeld * blockDim.x; c < cols; c += blockDim.x) s = fmaf(row[c], row[c], s);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
@@ -251,7 +261,12 @@ rmsnorm_kernel(const float* __restrict__ x, const float* __restrict__ w, float* 
   __syncthreads();
   const float gain = red[0];
   float* out = y + static_cast<size_t>(blockIdx.x) * cols;
-  for (int c = threadIdx.x; c < cols; c += blockDim.x) out[c] = row[c] * gain * w[c];
+#pragma unroll
+  for (int i = 0; i < kHeld; ++i) {
+    const int c = threadIdx.x + i * blockDim.x;
+    if (c < cols) out[c] = held[i] * gain * weight[i];
+  }
+  for (int c = threadIdx.x + kHeld * blockDim.x; c < cols; c += blockDim.x) out[c] = row[c] * gain * w[c];
 }
 
 // Whether an elementwise step over n floats takes the four-wide kernel: from 64k elements on (below, a quarter of the

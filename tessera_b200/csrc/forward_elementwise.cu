@@ -8,6 +8,7 @@
 
 #include "codec.cuh"
 #include "launch.h"
+#include "router.cuh"
 #include "tessera_b200.h"
 
 namespace tsr {
@@ -715,51 +716,20 @@ __global__ void __launch_bounds__(1024) head_norm_rope_kernel(const HeadNormRope
 // indices; output row r reads input row row_base + r (src/backends/rocm/rocm_kernels.hpp:558-566).  One
 // CTA per row; top_k rounds of a block-wide arg-max over the values not taken yet; among equal values the
 // lowest index wins.
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kRouterThreads)
 top_k_rows_kernel(const float* __restrict__ logits, uint32_t* __restrict__ ids, float* __restrict__ vals, size_t vocab,
                   int top_k, size_t row_base) {
-  __shared__ float bv[8];
-  __shared__ uint32_t bi[8];
-  __shared__ uint32_t taken[32];
-  const float* row = logits + (row_base + blockIdx.x) * vocab;
-  for (int p = 0; p < top_k; ++p) {
-    float best = -INFINITY;
-    uint32_t arg = 0xFFFFFFFFu;
-    for (size_t c = threadIdx.x; c < vocab; c += blockDim.x) {
-      const float x = row[c];
-      bool used = false;
-      for (int t = 0; t < p; ++t) used = used || taken[t] == static_cast<uint32_t>(c);
-      if (!used && (x > best || (x == best && static_cast<uint32_t>(c) < arg) || arg == 0xFFFFFFFFu)) {
-        best = x;
-        arg = static_cast<uint32_t>(c);
-      }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ov = __shfl_xor_sync(0xFFFFFFFFu, best, o);
-      const uint32_t oi = __shfl_xor_sync(0xFFFFFFFFu, arg, o);
-      if (oi != 0xFFFFFFFFu && (arg == 0xFFFFFFFFu || ov > best || (ov == best && oi < arg))) {
-        best = ov;
-        arg = oi;
-      }
-    }
-    if ((threadIdx.x & 31) == 0) {
-      bv[threadIdx.x >> 5] = best;
-      bi[threadIdx.x >> 5] = arg;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      for (int x = 1; x < 8; ++x)
-        if (bi[x] != 0xFFFFFFFFu && (bi[0] == 0xFFFFFFFFu || bv[x] > bv[0] || (bv[x] == bv[0] && bi[x] < bi[0]))) {
-          bv[0] = bv[x];
-          bi[0] = bi[x];
-        }
-      taken[p] = bi[0];
-      vals[blockIdx.x * top_k + p] = bi[0] == 0xFFFFFFFFu ? -INFINITY : bv[0];
-      ids[blockIdx.x * top_k + p] = bi[0] == 0xFFFFFFFFu ? 0u : bi[0];
-    }
-    __syncthreads();
-  }
+  __shared__ TopKShared shared;
+  const size_t r = blockIdx.x;
+  top_k_block(logits + (row_base + r) * vocab, ids + r * top_k, vals + r * top_k, vocab, top_k, shared);
+}
+template <int P>
+__global__ void __launch_bounds__(kRouterThreads)
+top_k_small_kernel(const float* __restrict__ logits, uint32_t* __restrict__ ids, float* __restrict__ vals, int vocab,
+                   int top_k, size_t row_base) {
+  __shared__ TopKShared shared;
+  const size_t r = blockIdx.x;
+  top_k_small<P>(logits + (row_base + r) * vocab, ids + r * top_k, vals + r * top_k, vocab, top_k, shared, [] {});
 }
 
 unsigned blocks_of(size_t n) { return static_cast<unsigned>((n + 255) / 256); }
@@ -928,8 +898,13 @@ int tsr_conv1d_state(const float* qkv, const float* w, float* hist, float* q, fl
 int tsr_top_k_rows(const float* logits, uint32_t* ids, float* vals, uint64_t rows, uint64_t vocab, uint64_t top_k,
                    uint64_t row_base, void* stream) {
   if (!logits || !ids || !vals || !fits31(rows) || !fits31(vocab) || top_k == 0 || top_k > 32) return kInvalidArgument;
-  top_k_rows_kernel<<<static_cast<unsigned>(rows), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      logits, ids, vals, vocab, static_cast<int>(top_k), row_base);
+  auto st = static_cast<cudaStream_t>(stream);
+  const unsigned n = static_cast<unsigned>(rows);
+  const int cols = static_cast<int>(vocab), t = static_cast<int>(top_k);
+  if (vocab <= 128) top_k_small_kernel<4><<<n, kRouterThreads, 0, st>>>(logits, ids, vals, cols, t, row_base);
+  else if (vocab <= 256) top_k_small_kernel<8><<<n, kRouterThreads, 0, st>>>(logits, ids, vals, cols, t, row_base);
+  else if (vocab <= kTopKSmall) top_k_small_kernel<32><<<n, kRouterThreads, 0, st>>>(logits, ids, vals, cols, t, row_base);
+  else top_k_rows_kernel<<<n, kRouterThreads, 0, st>>>(logits, ids, vals, vocab, t, row_base);
   return check_launch();
 }
 

@@ -279,6 +279,11 @@ struct HeadNormRope {
   float* v_row;
 };
 int launch_head_norm_rope(const HeadNormRope& p, cudaStream_t st);
+// Mixture-of-experts layer: top_k_rows (one row) and moe_gate; moe_scale_add and the add of its result.
+int launch_router_select(const float* logits, uint32_t* ids, float* vals, const float* x, const float* w, float* wts, float* sig,
+                         uint64_t vocab, uint64_t top_k, uint64_t hidden, cudaStream_t st);
+int launch_moe_scale_add_add(const float* a, const float* b, const float* f, float* o, const float* base, float* out, uint64_t n,
+                             uint64_t idx, cudaStream_t st);
 // tsr_attention with out = attention * sigmoid(gate) written by the merge kernel (gate null: plain).
 int attention_gated(int kv_format, const float* q, const void* k, const void* v, const float* k_scale, const float* v_scale,
                     float* out, const float* gate, uint64_t m, uint64_t n, uint64_t heads, uint64_t kv_heads, uint64_t head_dim,

@@ -120,3 +120,54 @@ def test_expert_ids_beyond_the_tensors_are_refused_or_ignored(backend):
                              KernelLaunch(buffers=[backend.upload(x), small, backend.upload(up), backend.upload(ids), bphi],
                                           scalars=[hidden, inter, top_k, per, per]))
     backend.Synchronize()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("vocab,top_k", [(1, 1), (31, 8), (100, 32), (128, 8), (129, 3), (256, 8), (257, 32), (1000, 5), (1024, 32), (1025, 8)])
+def test_top_k_of_router_sized_rows(backend, oracle, vocab, top_k):
+    """Rows in registers (up to 1024 logits) and beyond: ties to the lowest index, minus infinities, all-equal rows."""
+    g = np.random.default_rng(vocab)
+    rows = 3
+    top_k = min(top_k, vocab)
+    logits = np.round(g.standard_normal((rows, vocab)) * 4).astype(np.float32) / 4     # many ties
+    logits[1] = 0.5
+    logits[2, : vocab // 2] = -np.inf
+    ib, vb = backend.AllocateBuffer(rows * top_k * 4), backend.AllocateBuffer(rows * top_k * 4)
+    backend.LaunchKernel(backend.LoadKernel("top_k_rows"), KernelLaunch(buffers=[backend.upload(logits), ib, vb], scalars=[rows, vocab, top_k, 0]))
+    ids, vals = oracle.top_k_rows(logits, rows, vocab, top_k)
+    assert np.array_equal(backend.download(ib, np.uint32, rows * top_k).reshape(rows, top_k), ids)
+    assert np.array_equal(backend.download(vb, np.float32, rows * top_k).reshape(rows, top_k), vals)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("experts,top_k,hidden", [(60, 4, 1024), (256, 8, 2048), (1024, 32, 768), (1500, 6, 512)])
+def test_merged_router_and_residual(backend, experts, top_k, hidden):
+    """top_k_rows + moe_gate and moe_scale_add + add queued side by side run as one launch each (where the row fits) and
+    give the separate launches' bits; an add that reads something else is left alone."""
+    g = np.random.default_rng(experts)
+    up, f = backend.upload, lambda n: backend.AllocateBuffer(n * 4)
+    logits, x, w = up(g.standard_normal(experts).astype(np.float32)), up(g.standard_normal(hidden).astype(np.float32)), up(g.standard_normal(hidden).astype(np.float32) * 0.05)
+    a, b, res = (up(g.standard_normal(hidden).astype(np.float32)) for _ in range(3))
+    L = lambda name, bufs, sc: backend.LaunchKernel(backend.LoadKernel(name), KernelLaunch(buffers=bufs, scalars=sc))
+
+    def issue():
+        out = [f(top_k), f(top_k), f(top_k), f(1), f(hidden), f(hidden), f(hidden)]
+        ids, vals, wts, sig, ff, x1, other = out
+        L("top_k_rows", [logits, ids, vals], [1, experts, top_k, 0])
+        L("moe_gate", [vals, x, w, wts, sig], [top_k, hidden])
+        L("moe_scale_add", [a, b, sig, ff], [hidden, 0])
+        L("add", [res, ff, x1], [hidden])
+        L("moe_scale_add", [a, b, sig, ff], [hidden, 0])
+        L("add", [res, a, other], [hidden])
+        backend.Synchronize()
+        return [backend.download(o, np.uint32, o.Size() // 4) for o in out]
+    want = issue()
+    backend.SetDeferred(2)
+    try:
+        before = backend.LaunchStats()[1]
+        got = issue()
+        kernels = backend.LaunchStats()[1] - before
+    finally:
+        backend.SetDeferred(0)
+    assert all(np.array_equal(x, y) for x, y in zip(got, want))
+    assert kernels == (4 if experts <= 1024 else 5)
