@@ -269,12 +269,12 @@ rmsnorm_kernel(const float* __restrict__ x, const float* __restrict__ w, float* 
   for (int c = threadIdx.x + kHeld * blockDim.x; c < cols; c += blockDim.x) out[c] = row[c] * gain * w[c];
 }
 
-// Whether an elementwise step over n floats takes the four-wide kernel: from 64k elements on (below, a quarter of the
+// Whether an elementwise step over n floats takes the four-wide kernel: from 256k elements on (below, a quarter of the
 // threads is a quarter of the SMs), whole and aligned, and with an output that is one of the inputs or apart from them (a
 // thread reads four elements before it writes four).
 static bool wide4(const float* a, const float* b, const float* o, uint64_t n) {
   auto apart = [&](const float* x) { return x == o || o + n <= x || x + n <= o; };
-  return n >= (1u << 16) && n % 4 == 0 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(o)) & 15u) == 0 &&
+  return n >= (1u << 18) && n % 4 == 0 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(o)) & 15u) == 0 &&
          apart(a) && apart(b);
 }
 static unsigned blocks_for(uint64_t n, unsigned per) {

@@ -274,7 +274,7 @@ def test_head_sized_rows(backend, oracle, rows, cols):
     assert np.all(y[:3] == np.float32(-3e9)) and np.all(y[-4:] == np.float32(-3e9))
 
 
-@pytest.mark.parametrize("n", [1 << 16, (1 << 16) + 4, (1 << 16) + 1, 65532])
+@pytest.mark.parametrize("n", [1 << 18, (1 << 18) + 4, (1 << 18) + 1, (1 << 18) - 4])
 def test_wide_elementwise_steps(backend, oracle, n):
     """silu_mul and add on both sides of the four-wide kernels' limit, and in place."""
     g = np.random.default_rng(n)
