@@ -407,8 +407,9 @@ int run_attention(int kvkind, const float* q, const void* k, const void* v, cons
   AttnParams p;
   if (int rc = check_attention(kvkind, q, k, v, ks, vs, m, n, heads, kv_heads, head_dim, q_base, row_base, window, causal, 1, &p))
     return rc;
-  const int tile = attention_tile(kvkind, p, out, gate, st);
-  if (tile != kUnsupportedFeature) return tile;
+  int rc = attention_tile(kvkind, p, out, gate, st);
+  if (rc == kUnsupportedFeature) rc = attention_few(kvkind, p, out, gate, st);
+  if (rc != kUnsupportedFeature) return rc;
   // as many chunks as keep a CTA busy with kAttnMinKeys keys, counted on the longest row's range
   const uint64_t span = window != 0 && window < n ? window : n;
   uint64_t splits = span / kAttnMinKeys;
@@ -422,7 +423,8 @@ int run_attention(int kvkind, const float* q, const void* k, const void* v, cons
   p.pacc = reinterpret_cast<float*>(scratch);
   p.pmax = reinterpret_cast<float*>(scratch + acc_bytes);
   p.psum = reinterpret_cast<float*>(scratch + acc_bytes + stat_bytes);
-  if (int rc = run_split(kvkind, p, st)) return rc;
+  rc = run_split(kvkind, p, st);
+  if (rc != kOk) return rc;
   return run_combine(p.pacc, p.pmax, p.psum, out, gate, m, heads, head_dim, splits, row_base, st);
 }
 

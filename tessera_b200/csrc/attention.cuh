@@ -40,4 +40,7 @@ struct AttnParams {
 // 16-bit and narrower caches, out = attention [* sigmoid(gate)].  kUnsupportedFeature: not one of its shapes.
 int attention_tile(int kvkind, AttnParams p, float* out, const float* gate, cudaStream_t st);
 
+// The same of a few rows over an FP8, int8 or 4-bit cache.
+int attention_few(int kvkind, AttnParams p, float* out, const float* gate, cudaStream_t st);
+
 }  // namespace tsr

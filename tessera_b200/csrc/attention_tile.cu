@@ -21,6 +21,8 @@
 // 24 heads of 256: 394 us against 4470 (123 TFLOP/s of the contract's 48 GFLOP, 246 of the MMAs').
 #include <cuda_fp16.h>
 
+#include <atomic>
+
 #include "attention.cuh"
 #include "codec.cuh"
 #include "launch.h"
@@ -137,6 +139,62 @@ __device__ __forceinline__ void key_range(const AttnParams& p, int i, int& start
 
 __device__ __forceinline__ float gated(float v, const float* gate, size_t at) {
   return gate != nullptr ? v / (1.0f + expf(-gate[at])) : v;
+}
+
+// Rows [row0, row0 + rows) of kv head `kv` over keys [c0, c1), a warp per row and key by key in fp32: for chunks that hold
+// infinities or NaN.  The result goes to `acc_s` / `top_s` (base-2 exponent) / `total_s` by row, or is `out` itself, or the
+// partial of chunk `split`.
+template <int KV, int D>
+__device__ __noinline__ void scalar_rows(const AttnParams& p, int kv, int group, int row0, int rows, int c0, int c1, int split,
+                                         int warp, int warps, float* out, const float* gate, float* acc_s, float* top_s, float* total_s) {
+  constexpr bool kScaled = KV >= kKvFp8;
+  constexpr int kRowBytes = D * kv_bits<KV>() / 8;
+  const int lane = threadIdx.x & 31;
+  const size_t row_bytes = static_cast<size_t>(p.kv_heads) * kRowBytes;
+  const unsigned char* kbase = static_cast<const unsigned char*>(p.k) + static_cast<size_t>(kv) * kRowBytes;
+  const unsigned char* vbase = static_cast<const unsigned char*>(p.v) + static_cast<size_t>(kv) * kRowBytes;
+  for (int r = warp; r < rows; r += warps) {
+    const int i = (row0 + r) / group, g = (row0 + r) - i * group;
+    const size_t head_row = (p.row_base + i) * p.heads + static_cast<size_t>(kv) * group + g;
+    int s0, l0;
+    key_range(p, i, s0, l0);
+    float x[D / 32], acc[D / 32];
+#pragma unroll
+    for (int e = 0; e < D / 32; ++e) x[e] = p.q[head_row * D + e * 32 + lane] * (kLog2e / sqrtf(static_cast<float>(D))), acc[e] = 0.0f;
+    float top = kNoKey, total = 0.0f;
+    for (int j = max(s0, c0); j < min(l0 + 1, c1); ++j) {
+      const unsigned char *kr = kbase + j * row_bytes, *vr = vbase + j * row_bytes;
+      float dot = 0.0f;
+#pragma unroll
+      for (int e = 0; e < D / 32; ++e) dot = fmaf(x[e], cache_element<KV>(kr, e * 32 + lane), dot);
+      const float sc = warp_sum(dot) * (kScaled ? p.ks[j] : 1.0f);
+      if (sc > top) {
+        const float corr = exp2f(top - sc);
+        total *= corr;
+#pragma unroll
+        for (int e = 0; e < D / 32; ++e) acc[e] *= corr;
+        top = sc;
+      }
+      const float w = exp2f(sc - top);
+      total += w;
+#pragma unroll
+      for (int e = 0; e < D / 32; ++e) acc[e] = fmaf(w * (kScaled ? p.vs[j] : 1.0f), cache_element<KV>(vr, e * 32 + lane), acc[e]);
+    }
+    const size_t at = head_row * D;
+    const size_t part = (static_cast<size_t>(i) * p.heads + static_cast<size_t>(kv) * group + g) * p.splits + split;
+#pragma unroll
+    for (int e = 0; e < D / 32; ++e) {
+      if (acc_s != nullptr) acc_s[r * D + e * 32 + lane] = acc[e];
+      else if (out != nullptr) out[at + e * 32 + lane] = gated(acc[e] / total, gate, at + e * 32 + lane);
+      else p.pacc[part * D + e * 32 + lane] = acc[e];
+    }
+    if (acc_s != nullptr) {
+      if (lane == 0) top_s[r] = top, total_s[r] = total;
+    } else if (out == nullptr && lane == 0) {
+      p.pmax[part] = top == kNoKey && total == 0.0f ? kNullMax : top * kLn2;
+      p.psum[part] = total;
+    }
+  }
 }
 
 // grid: (kv_heads * row_tiles, splits).  Shared memory: the queries' two terms, one tile of keys and one of values in
@@ -468,48 +526,9 @@ __global__ void __launch_bounds__(kTileThreads, 1) attention_tile_kernel(const A
   cp_async_wait<0>();
 
   const size_t chunk_stride = static_cast<size_t>(p.splits);
-  if (any_bad) {
-    // Infinities or NaN somewhere in the chunk: a two-term product of them is not the product, and a masked key's
-    // zero weight would not mask them.  The whole chunk again, a warp per row and key by key in fp32.
-    for (int r = warp; r < rows; r += kTileThreads / 32) {
-      const int i = (row0 + r) / group, g = (row0 + r) - i * group;
-      const size_t head_row = (p.row_base + i) * p.heads + static_cast<size_t>(kv) * group + g;
-      int s0, l0;
-      key_range(p, i, s0, l0);
-      float x[D / 32], acc[D / 32];
-#pragma unroll
-      for (int e = 0; e < D / 32; ++e) x[e] = p.q[head_row * D + e * 32 + lane] * (kLog2e / sqrtf(static_cast<float>(D))), acc[e] = 0.0f;
-      float top = kNoKey, total = 0.0f;
-      for (int j = max(s0, c0); j < min(l0 + 1, c1); ++j) {
-        const unsigned char *kr = kbase + j * row_bytes, *vr = vbase + j * row_bytes;
-        float dot = 0.0f;
-#pragma unroll
-        for (int e = 0; e < D / 32; ++e) dot = fmaf(x[e], cache_element<KV>(kr, e * 32 + lane), dot);
-        const float sc = warp_sum(dot) * (kScaled ? p.ks[j] : 1.0f);
-        if (sc > top) {
-          const float corr = exp2f(top - sc);
-          total *= corr;
-#pragma unroll
-          for (int e = 0; e < D / 32; ++e) acc[e] *= corr;
-          top = sc;
-        }
-        const float w = exp2f(sc - top);
-        total += w;
-#pragma unroll
-        for (int e = 0; e < D / 32; ++e) acc[e] = fmaf(w * (kScaled ? p.vs[j] : 1.0f), cache_element<KV>(vr, e * 32 + lane), acc[e]);
-      }
-      const size_t at = head_row * D;
-      const size_t part = (static_cast<size_t>(i) * p.heads + static_cast<size_t>(kv) * group + g) * chunk_stride + split;
-#pragma unroll
-      for (int e = 0; e < D / 32; ++e) {
-        if (tp.out != nullptr) tp.out[at + e * 32 + lane] = gated(acc[e] / total, tp.gate, at + e * 32 + lane);
-        else p.pacc[part * D + e * 32 + lane] = acc[e];
-      }
-      if (tp.out == nullptr && lane == 0) {
-        p.pmax[part] = top == kNoKey && total == 0.0f ? kNullMax : top * kLn2;
-        p.psum[part] = total;
-      }
-    }
+  if (any_bad) {  // a two-term product with an infinity or NaN is not the product, and a masked key's zero weight would not mask it
+    scalar_rows<KV, D>(p, kv, group, row0, rows, c0, c1, split, warp, kTileThreads / 32, tp.out, tp.gate, nullptr, nullptr,
+                         nullptr);
     return;
   }
   if (!active) return;
@@ -539,6 +558,375 @@ __global__ void __launch_bounds__(kTileThreads, 1) attention_tile_kernel(const A
       }
     }
   }
+}
+
+// ---- few rows (a decoded token, two or three drafted ones) ----
+// The chunk kernel of attention.cu is bound by its instructions (about 1000 for four keys of a warp), and its chunks meet
+// in a second launch.  Here a cluster of up to sixteen CTAs takes one kv head and 8 NT (row, head) pairs over the whole key
+// range: a CTA a chunk, a warp sixteen keys at a time, and the chunks meet through distributed shared memory.
+// The products are S^T = K Q^T and O^T = V^T P^T, so that eight rows fill an MMA.  Keys and values go from global memory
+// to MMA fragments in registers without shared memory, because the order of the elements along a contraction and of the
+// output rows is free: lane t of a key's four reads 16-byte pieces t, t + 4, ... of its row, and the queries are laid out in
+// that order; lane g of a value's eight reads the g-th eighth of its row.  The weights come out of the score MMA with keys
+// along g and are turned by movmatrix.  Two terms per query element and weight and exact cache elements as above; sixteen
+// keys' weights are normalised by their largest value scale.
+constexpr int kFewWarps = 8, kFewKeys = 16, kFewCluster = 16;
+#ifndef FEWC
+#define FEWC 16
+#endif
+#ifndef FEWG
+#define FEWG 4
+#endif
+#ifndef FEWW
+#define FEWW 64
+#endif
+
+template <int KV, int D, int NT>
+struct FewShape {
+  static constexpr int kRows = 8 * NT, kRowBytes = D * kv_bits<KV>() / 8;
+  static constexpr int kPiece = 128 / kv_bits<KV>();               // elements of a 16-byte piece
+  static constexpr int kKeyPieces = kRowBytes / 64;                // of a key row, per lane
+  static constexpr int kValueWords = kRowBytes / 32;               // 32-bit words of a value row, per lane
+  static constexpr int kEighth = D / 8 + 2, kPitch = 8 * kEighth + 4;  // of a row's sums: 8-byte stores without conflicts
+  static constexpr int kQBytes = 2 * kRows * D * 2, kAccBytes = kRows * D * 4;
+  static constexpr int kSmem = kQBytes + kAccBytes + kFewWarps * kRows * (kPitch + 2) * 4 + 4 * kRows * 4;
+};
+
+__device__ __forceinline__ uint32_t transpose_8x8(uint32_t v) {
+  uint32_t r;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t local, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float ld_cluster(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+
+// grid: (kv_heads * splits, row tiles) in clusters of (splits, 1)
+template <int KV, int D, int NT>
+__global__ void __launch_bounds__(kFewWarps * 32, 1) attention_few_kernel(const AttnParams p, int group, float* out, const float* gate) {
+  using S = FewShape<KV, D, NT>;
+  static_assert(kv_bits<KV>() <= 8, "formats with a scale per row");
+  constexpr int kWordSteps = kv_bits<KV>() == 8 ? 1 : 2;  // k steps a 32-bit word of a key feeds
+  constexpr int kPer = 32 / kv_bits<KV>();                // elements of a word
+  constexpr int kGroup = FEWG;  // MMA pairs in flight: the second of a pair waits for the first
+  constexpr int kRows = S::kRows;
+  extern __shared__ __align__(128) unsigned char smem[];
+  uint32_t* const q_s = reinterpret_cast<uint32_t*>(smem);                 // [D / 16][NT][hi, lo][32 lanes][2]
+  float* const acc_s = reinterpret_cast<float*>(smem + S::kQBytes);        // [rows][D], the CTA's sums
+  float* const part = acc_s + kRows * D;                                   // [warps][rows][kPitch]
+  float* const wmax = part + kFewWarps * kRows * S::kPitch;                // [warps][rows]
+  float* const wsum = wmax + kFewWarps * kRows;
+  float* const top_s = wsum + kFewWarps * kRows;                           // [rows], the CTA's
+  float* const total_s = top_s + kRows;
+  float* const row_f = total_s + kRows;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int kv = blockIdx.x / p.splits, split = blockIdx.x - kv * p.splits;
+  const int row0 = blockIdx.y * kRows, rows = min(kRows, p.m * group - row0);
+  int first, last, unused;
+  key_range(p, row0 / group, first, unused);
+  key_range(p, (row0 + rows - 1) / group, unused, last);
+  const int keys = last - first + 1, chunk = (keys + p.splits - 1) / p.splits;
+  const int c0 = first + split * chunk, c1 = min(last + 1, c0 + chunk);
+  const unsigned char* kbase = static_cast<const unsigned char*>(p.k) + static_cast<size_t>(kv) * S::kRowBytes;
+  const unsigned char* vbase = static_cast<const unsigned char*>(p.v) + static_cast<size_t>(kv) * S::kRowBytes;
+  const size_t row_bytes = static_cast<size_t>(p.kv_heads) * S::kRowBytes;
+  bool bad = false;
+
+  uint32_t kraw[2][S::kKeyPieces][4], vraw[4][S::kValueWords];
+  float ksc[2], vsc[2];  // of keys base + g and base + 8 + g
+  auto load_keys = [&](int base) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int j = min(base + h * 8 + g, c1 - 1);
+      const unsigned char* row = kbase + j * row_bytes;
+#pragma unroll
+      for (int u = 0; u < S::kKeyPieces; ++u) {
+        const uint4 x = __ldg(reinterpret_cast<const uint4*>(row + (u * 4 + t) * 16));
+        kraw[h][u][0] = x.x, kraw[h][u][1] = x.y, kraw[h][u][2] = x.z, kraw[h][u][3] = x.w;
+      }
+      ksc[h] = __ldg(p.ks + j), vsc[h] = __ldg(p.vs + j);
+    }
+  };
+  auto load_values = [&](int base) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int j = min(base + 2 * t + (u & 1) + 8 * (u >> 1), c1 - 1);
+      const unsigned char* row = vbase + j * row_bytes + g * (S::kRowBytes / 8);
+      if constexpr (S::kValueWords >= 4) {
+#pragma unroll
+        for (int x4 = 0; x4 < S::kValueWords / 4; ++x4) {
+          const uint4 x = __ldg(reinterpret_cast<const uint4*>(row) + x4);
+          vraw[u][4 * x4] = x.x, vraw[u][4 * x4 + 1] = x.y, vraw[u][4 * x4 + 2] = x.z, vraw[u][4 * x4 + 3] = x.w;
+        }
+      } else {
+        const uint2 x = __ldg(reinterpret_cast<const uint2*>(row));
+        vraw[u][0] = x.x, vraw[u][1] = x.y;
+      }
+    }
+  };
+  const int begin = c0 + warp * kFewKeys;
+  if (begin < c1) {
+    load_keys(begin);
+    load_values(begin);
+  }
+
+  // queries in fragment order, scaled as in the tile kernel: a warp per row
+  const float q_scale = kLog2e / sqrtf(static_cast<float>(D));
+#pragma unroll
+  for (int u = 0; u < NT; ++u) {
+    const int r = u * 8 + warp, i = (row0 + r) / group, hd = (row0 + r) - i * group;
+    const float* src = p.q + ((p.row_base + i) * p.heads + static_cast<size_t>(kv) * group + hd) * D + lane * 4;
+    float4 x[D / 128];
+    float top = 0.0f;
+#pragma unroll
+    for (int it = 0; it < D / 128; ++it) {
+      float4 y = r < rows ? __ldg(reinterpret_cast<const float4*>(src + it * 128)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      y = make_float4(y.x * q_scale, y.y * q_scale, y.z * q_scale, y.w * q_scale);
+      bad |= !(fabsf(y.x) <= 3.402823466e38f) || !(fabsf(y.y) <= 3.402823466e38f) || !(fabsf(y.z) <= 3.402823466e38f) ||
+             !(fabsf(y.w) <= 3.402823466e38f);
+      top = fmaxf(top, fmaxf(fmaxf(fabsf(y.x), fabsf(y.y)), fmaxf(fabsf(y.z), fabsf(y.w))));
+      x[it] = y;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xFFFFFFFFu, top, o));
+    int e = static_cast<int>((__float_as_uint(top) >> 23) & 0xFFu) - 127 - 13;
+    e = max(-110, min(114, e));
+    if (top == 0.0f) e = 0;
+    const float upf = __uint_as_float(static_cast<uint32_t>(127 - e) << 23);
+    if (lane == 0) row_f[r] = __uint_as_float(static_cast<uint32_t>(127 + e) << 23);
+#pragma unroll
+    for (int it = 0; it < D / 128; ++it) {
+      // elements d .. d + 3 are one lane's four of a k step: piece j = d / (4 kPiece), lane (d / kPiece) % 4
+      const int d = it * 128 + lane * 4, j = d / (4 * S::kPiece), tq = (d / S::kPiece) & 3, step = j * (S::kPiece / 4) + (d % S::kPiece) / 4;
+      uint2 hi, lo;
+      split_half2(x[it].x * upf, x[it].y * upf, hi.x, lo.x);
+      split_half2(x[it].z * upf, x[it].w * upf, hi.y, lo.y);
+      uint2* const dst = reinterpret_cast<uint2*>(q_s) + (step * NT + u) * 64 + warp * 4 + tq;
+      dst[0] = hi, dst[32] = lo;
+    }
+  }
+  __syncthreads();
+
+  int start[NT][2], stop[NT][2];  // of rows 8 nt + 2t and + 1, the rows of this lane's scores and sums
+  float rf[NT][2], mx[NT][2], sum[NT][2];
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int r = nt * 8 + 2 * t + u;
+      int s0 = 0, l0 = -1;
+      if (r < rows) key_range(p, (row0 + r) / group, s0, l0);
+      start[nt][u] = s0, stop[nt][u] = min(l0 + 1, c1);
+      rf[nt][u] = row_f[r], mx[nt][u] = kNoKey, sum[nt][u] = 0.0f;
+    }
+  float o[NT][D / 16][4];
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+    for (int j = 0; j < D / 16; ++j) o[nt][j][0] = o[nt][j][1] = o[nt][j][2] = o[nt][j][3] = 0.0f;
+  for (int base = begin; base < c1; base += kFewWarps * kFewKeys) {
+    const bool more = base + kFewWarps * kFewKeys < c1;
+    float s[NT][4];
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.0f;
+#pragma unroll
+    for (int w0 = 0; w0 < 4 * S::kKeyPieces; w0 += kGroup / kWordSteps) {
+      uint32_t b[2][kGroup / kWordSteps][2 * kWordSteps];
+      float pt[kGroup][NT][4] = {};
+#pragma unroll
+      for (int x = 0; x < kGroup / kWordSteps; ++x) {
+        bad |= expand_word<KV>(kraw[0][(w0 + x) / 4][(w0 + x) % 4], b[0][x]);
+        bad |= expand_word<KV>(kraw[1][(w0 + x) / 4][(w0 + x) % 4], b[1][x]);
+      }
+#pragma unroll
+      for (int lo = 1; lo >= 0; --lo)
+#pragma unroll
+        for (int x = 0; x < kGroup; ++x) {
+          const int wd = x / kWordSteps, h = 2 * (x % kWordSteps);
+          const uint32_t a[4] = {b[0][wd][h], b[1][wd][h], b[0][wd][h + 1], b[1][wd][h + 1]};
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt) {
+            const uint2 f = *reinterpret_cast<const uint2*>(q_s + (((w0 * kWordSteps + x) * NT + nt) * 64 + lo * 32 + lane) * 2);
+            mma_f16(pt[x][nt], a, f.x, f.y);
+          }
+        }
+#pragma unroll
+      for (int x = 0; x < kGroup; ++x)
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) s[nt][c] += pt[x][nt][c];
+    }
+    const float ks0 = ksc[0], ks1 = ksc[1], vs0 = vsc[0], vs1 = vsc[1];
+    if (more) load_keys(base + kFewWarps * kFewKeys);
+    bad |= !(fabsf(ks0) <= 3.402823466e38f) || !(fabsf(ks1) <= 3.402823466e38f) || !(fabsf(vs0) <= 3.402823466e38f) ||
+           !(fabsf(vs1) <= 3.402823466e38f);
+    float vtop = fmaxf(fabsf(vs0), fabsf(vs1));
+#pragma unroll
+    for (int x = 4; x < 32; x <<= 1) vtop = fmaxf(vtop, __shfl_xor_sync(0xFFFFFFFFu, vtop, x));
+    int ev = static_cast<int>((__float_as_uint(vtop) >> 23) & 0xFFu) - 127;
+    ev = max(-100, min(100, ev));
+    if (vtop == 0.0f) ev = 0;
+    const float v_norm = __uint_as_float(static_cast<uint32_t>(127 + kWeightBits - ev) << 23);
+    const float v_unit = __uint_as_float(static_cast<uint32_t>(127 - kWeightBits + ev) << 23);
+    uint32_t ph[NT][2], pl[NT][2];
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+      float corr[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int j = base + g;
+        const float x0 = s[nt][u] * (rf[nt][u] * ks0), x1 = s[nt][2 + u] * (rf[nt][u] * ks1);
+        s[nt][u] = (j >= start[nt][u] && j < stop[nt][u]) ? x0 : kNoKey;
+        s[nt][2 + u] = (j + 8 >= start[nt][u] && j + 8 < stop[nt][u]) ? x1 : kNoKey;
+        float top = fmaxf(s[nt][u], s[nt][2 + u]);
+#pragma unroll
+        for (int x = 4; x < 32; x <<= 1) top = fmaxf(top, __shfl_xor_sync(0xFFFFFFFFu, top, x));
+        const float now = fmaxf(mx[nt][u], top);
+        corr[u] = exp2f(mx[nt][u] - now);
+        mx[nt][u] = now;
+        s[nt][u] = s[nt][u] == kNoKey ? 0.0f : exp2f(s[nt][u] - now);
+        s[nt][2 + u] = s[nt][2 + u] == kNoKey ? 0.0f : exp2f(s[nt][2 + u] - now);
+        sum[nt][u] = fmaf(sum[nt][u], corr[u], s[nt][u] + s[nt][2 + u]);
+      }
+      if (__any_sync(0xFFFFFFFFu, corr[0] != 1.0f || corr[1] != 1.0f)) {
+#pragma unroll
+        for (int j = 0; j < D / 16; ++j)
+          o[nt][j][0] *= corr[0], o[nt][j][1] *= corr[1], o[nt][j][2] *= corr[0], o[nt][j][3] *= corr[1];
+      }
+      const float f0 = vs0 * v_norm, f1 = vs1 * v_norm;
+      split_half2(s[nt][0] * f0, s[nt][1] * f0, ph[nt][0], pl[nt][0]);
+      split_half2(s[nt][2] * f1, s[nt][3] * f1, ph[nt][1], pl[nt][1]);
+      ph[nt][0] = transpose_8x8(ph[nt][0]), ph[nt][1] = transpose_8x8(ph[nt][1]);
+      pl[nt][0] = transpose_8x8(pl[nt][0]), pl[nt][1] = transpose_8x8(pl[nt][1]);
+    }
+#pragma unroll
+    for (int w0 = 0; w0 < S::kValueWords; w0 += 2 * kGroup / kPer) {
+      uint32_t b[2][2 * kGroup];  // keys 2t, 2t + 1 of an element; keys 2t + 8, 2t + 9
+#pragma unroll
+      for (int wd = 0; wd < 2 * kGroup / kPer; ++wd)
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          const uint32_t wa = vraw[2 * half][w0 + wd], wb = vraw[2 * half + 1][w0 + wd];
+          uint32_t* const dst = b[half] + wd * kPer;
+          if constexpr (kv_bits<KV>() == 8) {
+            uint32_t x[2], y[2];
+            bad |= expand_word<KV>(__byte_perm(wa, wb, 0x5140), x);
+            bad |= expand_word<KV>(__byte_perm(wa, wb, 0x7362), y);
+            dst[0] = x[0], dst[1] = x[1], dst[2] = y[0], dst[3] = y[1];
+          } else {  // the two keys' nibbles of an element side by side
+            uint32_t x[4], y[4];
+            expand_word<KV>((wa & 0x0F0F0F0Fu) | ((wb & 0x0F0F0F0Fu) << 4), x);
+            expand_word<KV>(((wa >> 4) & 0x0F0F0F0Fu) | (wb & 0xF0F0F0F0u), y);
+#pragma unroll
+            for (int x4 = 0; x4 < 4; ++x4) dst[2 * x4] = x[x4], dst[2 * x4 + 1] = y[x4];
+          }
+        }
+      float pt[kGroup][NT][4] = {};
+#pragma unroll
+      for (int lo = 1; lo >= 0; --lo)
+#pragma unroll
+        for (int x = 0; x < kGroup; ++x) {
+          const uint32_t a[4] = {b[0][2 * x], b[0][2 * x + 1], b[1][2 * x], b[1][2 * x + 1]};
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt) {
+            if (lo) mma_f16(pt[x][nt], a, pl[nt][0], pl[nt][1]);
+            else mma_f16(pt[x][nt], a, ph[nt][0], ph[nt][1]);
+          }
+        }
+#pragma unroll
+      for (int x = 0; x < kGroup; ++x)
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            float& sum_o = o[nt][w0 * kPer / 2 + x][c];
+            sum_o = fmaf(pt[x][nt][c], v_unit, sum_o);
+          }
+    }
+    if (more) load_values(base + kFewWarps * kFewKeys);
+  }
+  if (__syncthreads_or(bad)) {
+    scalar_rows<KV, D>(p, kv, group, row0, rows, c0, c1, split, warp, kFewWarps, nullptr, nullptr, acc_s, top_s, total_s);
+  } else {
+    // the warps meet: the CTA's max per row, every warp's share rescaled to it, summed in warp order
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+#pragma unroll
+        for (int x = 4; x < 32; x <<= 1) sum[nt][u] += __shfl_xor_sync(0xFFFFFFFFu, sum[nt][u], x);
+        if (g == 0) wmax[warp * kRows + nt * 8 + 2 * t + u] = mx[nt][u];
+      }
+    __syncthreads();
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int r = nt * 8 + 2 * t + u;
+        float top = wmax[r];
+#pragma unroll
+        for (int w = 1; w < kFewWarps; ++w) top = fmaxf(top, wmax[w * kRows + r]);
+        const float f = exp2f(mx[nt][u] - top);  // 0 for a warp that had no key (1 when none had: its sums are 0)
+        if (g == 0) wsum[warp * kRows + r] = sum[nt][u] * f;
+        float* dst = part + (warp * kRows + r) * S::kPitch + g * S::kEighth;
+#pragma unroll
+        for (int j = 0; j < D / 16; ++j) *reinterpret_cast<float2*>(dst + 2 * j) = make_float2(o[nt][j][u] * f, o[nt][j][2 + u] * f);
+      }
+    __syncthreads();
+    for (int x = tid; x < rows * D; x += kFewWarps * 32) {
+      const int r = x / D, d = x - r * D;
+      const float* src = part + r * S::kPitch + d / (D / 8) * S::kEighth + d % (D / 8);
+      float total = 0.0f;
+#pragma unroll
+      for (int w = 0; w < kFewWarps; ++w) total += src[w * kRows * S::kPitch];
+      acc_s[x] = total;
+    }
+    if (tid < rows) {
+      float top = wmax[tid], total = 0.0f;
+#pragma unroll
+      for (int w = 1; w < kFewWarps; ++w) top = fmaxf(top, wmax[w * kRows + tid]);
+#pragma unroll
+      for (int w = 0; w < kFewWarps; ++w) total += wsum[w * kRows + tid];
+      top_s[tid] = top, total_s[tid] = total;
+    }
+  }
+  // the chunks meet: CTA `split` merges its share of the elements, all CTAs' values in flight
+  cluster_sync();
+  const int share = (rows * D + p.splits - 1) / p.splits;
+  for (int x = split * share + tid; x < min(rows * D, (split + 1) * share); x += kFewWarps * 32) {
+    const int r = x / D, d = x - r * D, i = (row0 + r) / group, hd = (row0 + r) - i * group;
+    float tops[kFewCluster], totals[kFewCluster], accs[kFewCluster], top = kNoKey, num = 0.0f, den = 0.0f;
+#pragma unroll
+    for (int c = 0; c < kFewCluster; ++c)
+      if (c < p.splits) {
+        tops[c] = ld_cluster(cluster_addr(smem_addr(top_s + r), c));
+        totals[c] = ld_cluster(cluster_addr(smem_addr(total_s + r), c));
+        accs[c] = ld_cluster(cluster_addr(smem_addr(acc_s + x), c));
+      }
+#pragma unroll
+    for (int c = 0; c < kFewCluster; ++c)
+      if (c < p.splits) top = fmaxf(top, tops[c]);
+#pragma unroll
+    for (int c = 0; c < kFewCluster; ++c)
+      if (c < p.splits) {
+        const float w = exp2f(tops[c] - top);
+        num = fmaf(w, accs[c], num), den = fmaf(w, totals[c], den);
+      }
+    const size_t at = ((p.row_base + i) * p.heads + static_cast<size_t>(kv) * group + hd) * D + d;
+    out[at] = gated(num / den, gate, at);
+  }
+  cluster_sync();  // the others may still read this CTA's sums
 }
 
 // The chunks of a (row, head): a thread per four elements, chunks in order (attention_combine's arithmetic; that
@@ -580,13 +968,89 @@ int launch_tile_d(const AttnTileParams& tp, cudaStream_t st) {
   return tp.a.head_dim == 256 ? launch_tile<KV, 256>(tp, st) : launch_tile<KV, 128>(tp, st);
 }
 
+// kUnsupportedFeature where the device does not take clusters of that size (a partitioned GPU).
+template <int KV, int D, int NT>
+int launch_few_nt(AttnParams p, int group, float* out, const float* gate, cudaStream_t st) {
+  using S = FewShape<KV, D, NT>;
+  const auto kernel = &attention_few_kernel<KV, D, NT>;
+  if (int rc = allow_dynamic_smem(reinterpret_cast<const void*>(kernel), S::kSmem)) return rc;
+  static std::atomic<int> resident[64];  // per device: clusters of sixteen that run at a time, plus one; 0 not asked
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return kDeviceError;
+  cudaLaunchConfig_t config{};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  config.blockDim = dim3(kFewWarps * 32);
+  config.dynamicSmemBytes = S::kSmem;
+  config.stream = st;
+  config.attrs = attr;
+  config.numAttrs = 1;
+  if (resident[dev].load(std::memory_order_relaxed) == 0) {
+    int clusters = 0;
+    attr[0].val.clusterDim.x = kFewCluster;
+    config.gridDim = dim3(kFewCluster);
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&clusters, kernel, &config) != cudaSuccess) {
+      cudaGetLastError();
+      clusters = 0;
+    }
+    resident[dev].store(clusters + 1, std::memory_order_relaxed);
+  }
+  const int fit = resident[dev].load(std::memory_order_relaxed) - 1, row_tiles = (p.m * group + S::kRows - 1) / S::kRows;
+  if (fit == 0) return kUnsupportedFeature;
+  // A GPU holds few clusters of sixteen (the SMs of one GPC each), twice as many of eight and a rest: a second wave costs
+  // more than twice the keys per CTA.  2 rows x 4096 keys, 32 heads over 8 of 128: 303 us a pass in sixteens, 201 in eights.
+  if (p.splits == kFewCluster && p.kv_heads * row_tiles > fit) p.splits = kFewCluster / 2;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(p.splits);
+  config.gridDim = dim3(static_cast<unsigned>(p.kv_heads * p.splits), static_cast<unsigned>(row_tiles));
+  if (cudaLaunchKernelEx(&config, kernel, p, group, out, gate) != cudaSuccess) return kDeviceError;
+  return check_launch();
+}
+
+template <int KV>
+int launch_few(const AttnParams& p, int group, float* out, const float* gate, cudaStream_t st) {
+  if (p.m * group <= 8)
+    return p.head_dim == 256 ? launch_few_nt<KV, 256, 1>(p, group, out, gate, st) : launch_few_nt<KV, 128, 1>(p, group, out, gate, st);
+  return p.head_dim == 256 ? launch_few_nt<KV, 256, 2>(p, group, out, gate, st) : launch_few_nt<KV, 128, 2>(p, group, out, gate, st);
+}
+
 bool overlap(const void* a, size_t an, const void* b, size_t bn) {
   const auto *x = static_cast<const unsigned char*>(a), *y = static_cast<const unsigned char*>(b);
   return x < y + bn && y < x + an;
 }
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+// Whether the result may be written while other CTAs still read their queries and the cache.  In place over q is fine (a
+// CTA or cluster reads its own rows before it writes them); any other overlap stays with the chunk kernel, whose merge
+// starts when everything has been read.
+bool writes_apart(int kvkind, const AttnParams& p, const float* out, const float* gate) {
+  const size_t out_bytes = static_cast<size_t>(p.m) * p.heads * p.head_dim * 4;
+  const size_t cache_bytes = static_cast<size_t>(p.n) * p.kv_heads * p.head_dim * (kvkind == kKvF16 ? 4 : kvkind == kKvInt4 ? 1 : 2) / 2;
+  const float *rows_q = p.q + p.row_base * p.heads * p.head_dim, *rows_out = out + p.row_base * p.heads * p.head_dim;
+  const size_t scale_bytes = kvkind == kKvF16 ? 0 : static_cast<size_t>(p.n) * 4;
+  return !((rows_out != rows_q && overlap(rows_out, out_bytes, rows_q, out_bytes)) || overlap(rows_out, out_bytes, p.k, cache_bytes) ||
+           overlap(rows_out, out_bytes, p.v, cache_bytes) ||
+           (scale_bytes != 0 && (overlap(rows_out, out_bytes, p.ks, scale_bytes) || overlap(rows_out, out_bytes, p.vs, scale_bytes))) ||
+           (gate != nullptr && overlap(rows_out, out_bytes, gate + p.row_base * p.heads * p.head_dim, out_bytes)));
+}
+
 }  // namespace
+
+int attention_few(int kvkind, AttnParams p, float* out, const float* gate, cudaStream_t st) {
+  const int group = p.heads / p.kv_heads;
+  const long span = p.causal && p.window != 0 && p.window < p.n ? p.window : p.n;
+  if (kvkind < kKvFp8 || !aligned16(p.q) || !aligned16(p.k) || !aligned16(p.v) || !writes_apart(kvkind, p, out, gate))
+    return kUnsupportedFeature;
+  // a warp's sixteen keys in each CTA before another CTA joins
+  p.splits = 1;
+  while (p.splits < FEWC && p.splits * FEWW < span) p.splits *= 2;
+  switch (kvkind) {
+    case kKvFp8: return launch_few<kKvFp8>(p, group, out, gate, st);
+    case kKvInt8: return launch_few<kKvInt8>(p, group, out, gate, st);
+    default: return launch_few<kKvInt4>(p, group, out, gate, st);
+  }
+}
 
 int attention_tile(int kvkind, AttnParams p, float* out, const float* gate, cudaStream_t st) {
   const int group = p.heads / p.kv_heads;
@@ -603,18 +1067,7 @@ int attention_tile(int kvkind, AttnParams p, float* out, const float* gate, cuda
   if (kvkind == kKvF32 || p.m < 4 || static_cast<double>(p.m) * span * p.kv_heads * p.head_dim < 8.0e6 || !aligned16(p.q) ||
       !aligned16(p.k) || !aligned16(p.v) || !aligned16(out))
     return kUnsupportedFeature;
-  // With one chunk the result is written while other CTAs still read their queries and the cache.  In place over q is
-  // fine (a CTA reads its own rows before it writes them); any other overlap stays with the chunk kernel, whose merge
-  // starts when everything has been read.
-  const size_t out_bytes = static_cast<size_t>(p.m) * p.heads * p.head_dim * 4;
-  const size_t cache_bytes = static_cast<size_t>(p.n) * p.kv_heads * p.head_dim * (kvkind == kKvF16 ? 4 : kvkind == kKvInt4 ? 1 : 2) / 2;
-  const float *rows_q = p.q + p.row_base * p.heads * p.head_dim, *rows_out = out + p.row_base * p.heads * p.head_dim;
-  const size_t scale_bytes = kvkind == kKvF16 ? 0 : static_cast<size_t>(p.n) * 4;
-  if ((rows_out != rows_q && overlap(rows_out, out_bytes, rows_q, out_bytes)) || overlap(rows_out, out_bytes, p.k, cache_bytes) ||
-      overlap(rows_out, out_bytes, p.v, cache_bytes) ||
-      (scale_bytes != 0 && (overlap(rows_out, out_bytes, p.ks, scale_bytes) || overlap(rows_out, out_bytes, p.vs, scale_bytes))) ||
-      (gate != nullptr && overlap(rows_out, out_bytes, gate + p.row_base * p.heads * p.head_dim, out_bytes)))
-    return kUnsupportedFeature;
+  if (!writes_apart(kvkind, p, out, gate)) return kUnsupportedFeature;
   static const int sms = [] {
     int dev = 0, v = 0;
     cudaGetDevice(&dev);

@@ -239,6 +239,39 @@ def test_batches_on_the_tensor_pipe(backend, oracle, fmt, m, n, heads, kv_heads,
     assert near(y, r)
 
 
+# (m, n, heads, kv_heads, head_dim, q_base, window): one key, fewer keys than a warp's sixteen, a chunk that ends inside a
+# warp's keys, eight rows of the sixteen over two row tiles, a window whose first keys leave chunks empty for the last row,
+# 64 chunks, the last of them empty
+FEW = [(1, 1, 24, 4, 256, 0, 0), (1, 13, 8, 8, 128, 12, 0), (1, 1000, 8, 1, 128, 900, 0), (3, 333, 16, 2, 256, 330, 0),
+       (3, 500, 6, 1, 128, 450, 70), (1, 4097, 24, 4, 256, 4096, 0), (2, 64, 12, 4, 256, 70, 0)]
+
+
+@pytest.mark.parametrize("fmt", [2, 3, 4])
+@pytest.mark.parametrize("m,n,heads,kv_heads,head_dim,q_base,window", FEW)
+def test_few_rows_on_the_tensor_pipe(backend, oracle, fmt, m, n, heads, kv_heads, head_dim, q_base, window):
+    """One to three query rows (two binary16 terms per query element and weight, exact cache elements): fp32 rounding."""
+    g = np.random.default_rng(80 + fmt + n)
+    q = g.standard_normal((m, heads * head_dim)).astype(np.float32) * np.float32(10.0) ** g.integers(-3, 2, (m, 1)).astype(np.float32)
+    k, v, ks, vs = make_cache(g, fmt, n, kv_heads * head_dim)
+    y = device_attention(backend, fmt, q, k, v, ks, vs, m, n, heads, kv_heads, head_dim, q_base, window, True, row_base=1)
+    r = oracle.attention(fmt, q, k, v, m, n, heads, kv_heads, head_dim, q_base, window, True, ks, vs)
+    assert near(y, r)
+
+
+def test_few_rows_with_nonfinite_values(backend, oracle):
+    """Two rows of which only the second sees a key whose scale is infinite and a NaN value."""
+    g = np.random.default_rng(90)
+    m, n, heads, kv_heads, head_dim = 2, 200, 8, 2, 128
+    q = np.abs(g.standard_normal((m, heads * head_dim))).astype(np.float32)
+    k, v, ks, vs = make_cache(g, 4, n, kv_heads * head_dim)
+    v[n - 1] = 0x7F
+    ks[n - 1] = np.inf
+    y = device_attention(backend, 4, q, k, v, ks, vs, m, n, heads, kv_heads, head_dim, n - 2, 0, True)
+    r = oracle.attention(4, q, k, v, m, n, heads, kv_heads, head_dim, n - 2, 0, True, ks, vs).reshape(y.shape)
+    assert near(y[:1], r[:1])
+    assert np.isnan(y[1:]).all() and np.isnan(r[1:]).all()
+
+
 def test_batch_without_causal_mask(backend, oracle):
     g = np.random.default_rng(60)
     m, n, heads, kv_heads, head_dim = 320, 333, 8, 2, 128
