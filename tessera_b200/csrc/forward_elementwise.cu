@@ -735,6 +735,11 @@ top_k_small_kernel(const float* __restrict__ logits, uint32_t* __restrict__ ids,
 unsigned blocks_of(size_t n) { return static_cast<unsigned>((n + 255) / 256); }
 bool fits31(uint64_t v) { return v > 0 && v <= 0x7FFFFFFFull; }
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+struct Span {  // `count` floats from `p`
+  const float* p;
+  uint64_t count;
+  bool meets(const Span& o) const { return count != 0 && o.count != 0 && p < o.p + o.count && o.p < p + count; }
+};
 
 }  // namespace
 
@@ -887,7 +892,15 @@ int tsr_conv1d_state(const float* qkv, const float* w, float* hist, float* q, fl
     return kInvalidArgument;
   auto st = static_cast<cudaStream_t>(stream);
   const dim3 grid(blocks_of(conv_dim), static_cast<unsigned>((rows + kConvRows - 1) / kConvRows));
-  if (width == 4 && grid.y <= 65535)  // the width of the convolutions in use; others take their rows in turn
+  // The chunks of the row kernel run at the same time, so nothing it writes may lie over the input rows or the history
+  // it reads: in place (v over qkv where key_dim is 0) the rows go in turn.  Nor may hist_hist's slots lie over `hist`.
+  const uint64_t taps = conv_dim * (width - 1);
+  const Span in{qkv + qkv_offset, rows * conv_dim}, old{hist, taps};
+  const Span slots{hist_stride != 0 ? hist_hist + hist_stride : hist, hist_stride != 0 ? (rows - 1) * hist_stride + taps : 0};
+  bool apart = !in.meets(old) && !in.meets(slots) && !old.meets(slots);
+  for (const Span& out : {Span{q, rows * key_dim}, Span{k, rows * key_dim}, Span{v, rows * (conv_dim - 2 * key_dim)}})
+    apart = apart && !out.meets(in) && !out.meets(old);
+  if (width == 4 && grid.y <= 65535 && apart)  // the width of the convolutions in use; others take their rows in turn
     conv1d_rows_kernel<4><<<grid, 256, 0, st>>>(qkv, w, hist, q, k, v, hist_hist, conv_dim, key_dim, qkv_offset, rows, hist_stride);
   else
     conv1d_state_kernel<<<blocks_of(conv_dim), 256, 0, st>>>(qkv, w, hist, q, k, v, hist_hist, conv_dim, width, key_dim,

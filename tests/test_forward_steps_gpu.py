@@ -256,6 +256,21 @@ def test_conv1d_over_chunks_of_rows(backend, oracle, rows, history):
     test_conv1d_state(backend, oracle, rows, history)
 
 
+@pytest.mark.parametrize("rows", [1, 16, 700])
+def test_conv1d_in_place(backend, oracle, rows):
+    """No q and k columns and v over the input rows: each row is read before it is overwritten, by later rows too."""
+    g = np.random.default_rng(17 + rows)
+    conv_dim, width = 4096, 4
+    qkv = g.standard_normal(rows * conv_dim).astype(np.float32)
+    w = g.standard_normal(conv_dim * width).astype(np.float32)
+    hist = g.standard_normal(conv_dim * (width - 1)).astype(np.float32)
+    io, hb, none = backend.upload(qkv), backend.upload(hist), backend.AllocateBuffer(16)
+    run(backend, "conv1d_state", [io, backend.upload(w), hb, none, none, io, none], [conv_dim, width, 0, 0, rows, 0])
+    _, _, v, hist2, _ = oracle.conv1d_state(qkv, w, hist, conv_dim, width, 0, 0, rows, 0, None)
+    assert close(backend.download(io, np.float32, v.size), v, 2e-6)
+    assert np.array_equal(backend.download(hb, np.float32, hist.size), hist2)
+
+
 @pytest.mark.parametrize("rows,cols", [(1, 128), (9, 128), (9, 256), (17, 256)])
 def test_head_sized_rows(backend, oracle, rows, cols):
     """A warp per row: the last CTA partly filled, both widths, in place (l2norm) and with element bases (rmsnorm_gated)."""
