@@ -33,6 +33,7 @@ namespace {
 constexpr int kTileRows = 128, kTileKeys = 64, kTileThreads = 256;
 constexpr int kScoreChain = 1, kValueChain = 4;  // 16-wide k steps (of two MMAs) that share an accumulator
 constexpr int kWeightBits = 14;  // softmax weights (<= 1) and normalised value scales are stored times 2^14
+constexpr int kMinScaleExp = kWeightBits - 126;  // of a value scale: below, the power of two that takes it back would not be normal
 
 struct AttnTileParams {
   AttnParams a;
@@ -293,7 +294,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) attention_tile_kernel(const A
 #pragma unroll
     for (int w = 0; w < kTileThreads / 32; ++w) top = fmaxf(top, red[w]);
     int e = static_cast<int>((__float_as_uint(top) >> 23) & 0xFFu) - 127;
-    e = max(-100, min(100, e));
+    e = max(kMinScaleExp, min(127, e));
     if (top == 0.0f) e = 0;
     v_norm = __uint_as_float(static_cast<uint32_t>(127 + kWeightBits - e) << 23);
     v_unit = __uint_as_float(static_cast<uint32_t>(127 - kWeightBits + e) << 23);
@@ -775,7 +776,7 @@ __global__ void __launch_bounds__(kFewWarps * 32, 1) attention_few_kernel(const 
 #pragma unroll
     for (int x = 4; x < 32; x <<= 1) vtop = fmaxf(vtop, __shfl_xor_sync(0xFFFFFFFFu, vtop, x));
     int ev = static_cast<int>((__float_as_uint(vtop) >> 23) & 0xFFu) - 127;
-    ev = max(-100, min(100, ev));
+    ev = max(kMinScaleExp, min(127, ev));
     if (vtop == 0.0f) ev = 0;
     const float v_norm = __uint_as_float(static_cast<uint32_t>(127 + kWeightBits - ev) << 23);
     const float v_unit = __uint_as_float(static_cast<uint32_t>(127 - kWeightBits + ev) << 23);

@@ -26,6 +26,12 @@ def near(y, r):
     return float(np.max(np.abs(y - r))) <= TOL * float(np.max(np.abs(r)))
 
 
+def near_each(y, r, head_dim):
+    """`near` for every (row, head) by itself."""
+    y, r = y.reshape(-1, head_dim).astype(np.float64), r.reshape(-1, head_dim).astype(np.float64)
+    return bool(np.all(np.abs(y - r).max(1) <= TOL * np.abs(r).max(1)))
+
+
 def device_attention(backend, fmt, q, k, v, ks, vs, m, n, heads, kv_heads, head_dim, q_base, window, causal, row_base=0):
     width = heads * head_dim
     qfull = np.zeros((row_base + m, width), np.float32)
@@ -298,3 +304,27 @@ def test_nonfinite_values_reach_only_the_rows_that_see_them(backend, oracle, fmt
     clean = 250 - (n - m)
     assert near(y[:clean], r[:clean])
     assert np.isnan(y[clean:]).all() and np.isnan(r[clean:]).all()
+
+
+# (m, n, heads, kv_heads, head_dim) of both kernels: row tiles over few and many chunks and over one, a cluster of one and
+# of many CTAs with up to eight and up to sixteen rows
+SHAPES = [(22, 400, 24, 4, 256), (40, 4000, 16, 2, 128), (600, 64, 4, 2, 128), (1, 300, 16, 2, 256), (1, 60, 8, 2, 128),
+          (3, 1000, 24, 4, 128)]
+
+
+@pytest.mark.parametrize("fmt", [2, 3, 4])
+@pytest.mark.parametrize("exponent", [112, 103, -118])
+@pytest.mark.parametrize("m,n,heads,kv_heads,head_dim", SHAPES)
+def test_value_scales_at_the_ends_of_their_range(backend, oracle, fmt, exponent, m, n, heads, kv_heads, head_dim):
+    """Finite value scales near the largest and the smallest fp32 numbers give finite results."""
+    g = np.random.default_rng(110 + fmt + n)
+    q = g.standard_normal((m, heads * head_dim)).astype(np.float32)
+    k, v, ks, vs = make_cache(g, fmt, n, kv_heads * head_dim)
+    if fmt == 4:
+        v = np.where((v & 0x7F) > 0x40, v & 0xBF, v)      # |v| <= 2, so that the sums stay in range
+    q_base = max(0, n - m)
+    r = oracle.attention(fmt, q, k, v, m, n, heads, kv_heads, head_dim, q_base, 0, True, ks, vs)
+    factor = np.float32(2.0 ** (exponent + 7))            # vs is about 2^-7; a power of two changes nothing else
+    y = device_attention(backend, fmt, q, k, v, ks, vs * factor, m, n, heads, kv_heads, head_dim, q_base, 0, True)
+    assert np.isfinite(y).all()
+    assert near_each(y / factor, r, head_dim)
