@@ -9,7 +9,8 @@
 // so they run as m16n8k16 binary16 MMAs with fp32 accumulation.  Nothing is rounded to 16 bits on the way: cache
 // elements (FP8, int8, 4-bit, fp16) are exact in binary16, and a query element or a softmax weight enters as two
 // binary16 terms x = hi + lo of a value scaled by a power of two, 22 bits below the row's largest query element and
-// 2^-38 below the row's largest weight.  Scales of quantised rows multiply the score and the weight in fp32.  The MMA
+// 2^-38 below the row's largest weight of a tile.  Scales of quantised rows multiply the score and the weight in fp32, the
+// latter before it is split: what a row does not see, or hardly weighs, takes nothing from it.  The MMA
 // cuts off what falls below its accumulator instead of rounding (chains over 4096 keys came out 4e-6 off), so two MMAs
 // of a score and eight of an output share an accumulator, the small terms first, before it is added in fp32: 3.8e-7
 // against 64 bits where the chunk kernel's fp32 sums have 3.0e-7 (longer chains 4.9e-7 at 6 % less time).
@@ -32,8 +33,8 @@ namespace {
 
 constexpr int kTileRows = 128, kTileKeys = 64, kTileThreads = 256;
 constexpr int kScoreChain = 1, kValueChain = 4;  // 16-wide k steps (of two MMAs) that share an accumulator
-constexpr int kWeightBits = 14;  // softmax weights (<= 1) and normalised value scales are stored times 2^14
-constexpr int kMinScaleExp = kWeightBits - 126;  // of a value scale: below, the power of two that takes it back would not be normal
+constexpr int kWeightBits = 14;  // a row's largest weight (times its key's value scale) is stored in [2^14, 2^15)
+constexpr int kMinWeightExp = kWeightBits - 126;  // below, the power of two that takes it back would not be normal
 
 struct AttnTileParams {
   AttnParams a;
@@ -49,7 +50,7 @@ struct TileShape {
   static constexpr int kPieces = kTileKeys * kPiecesPerRow / kTileThreads;  // 16-byte pieces a thread moves per tile
   static constexpr int kQBytes = 2 * kTileRows * D * 2, kTileBytes = kTileKeys * D * 2;
   static constexpr int kRawBytes = KV == kKvF16 ? 0 : kTileKeys * kRowBytes;
-  static constexpr int kSmem = kQBytes + 2 * kTileBytes + 2 * kRawBytes + kTileRows * 4 + 2 * 2 * kTileKeys * 4 + 64;
+  static constexpr int kSmem = kQBytes + 2 * kTileBytes + 2 * kRawBytes + kTileRows * 4 + 2 * 2 * kTileKeys * 4;
 };
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
@@ -125,6 +126,13 @@ __device__ __forceinline__ float cache_element(const unsigned char* row, int e) 
   if (KV == kKvFp8) return e4m3_to_float(row[e]);
   if (KV == kKvInt8) return static_cast<float>(static_cast<signed char>(row[e]));
   return static_cast<float>(static_cast<int>(static_cast<uint32_t>(row[e >> 1]) << (28 - 4 * (e & 1))) >> 28);
+}
+
+// The power of two that takes a row's largest weight `most` to [2^14, 2^15), and its inverse.
+__device__ __forceinline__ void weight_unit(float most, float& up, float& unit) {
+  const int e = max(kMinWeightExp, static_cast<int>(__float_as_uint(most) >> 23) - 127);
+  up = __uint_as_float(static_cast<uint32_t>(127 + kWeightBits - e) << 23);
+  unit = __uint_as_float(static_cast<uint32_t>(127 - kWeightBits + e) << 23);
 }
 
 // The keys [start, last] query row i sees.
@@ -215,7 +223,6 @@ __global__ void __launch_bounds__(kTileThreads, 1) attention_tile_kernel(const A
   unsigned char* const v_raw = k_raw + S::kRawBytes;
   float* const row_f = reinterpret_cast<float*>(v_raw + S::kRawBytes);  // [128] score factor of a row
   float* const sc_s = row_f + kTileRows;                                 // [2 buffers][k, v][64] scales of a tile's keys
-  float* const red = sc_s + 4 * kTileKeys;                               // [8]
   const AttnParams& p = tp.a;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, group = tp.group;
   const int kv = blockIdx.x % p.kv_heads, rt = tp.row_tiles - 1 - static_cast<int>(blockIdx.x) / p.kv_heads, split = blockIdx.y;
@@ -277,28 +284,6 @@ __global__ void __launch_bounds__(kTileThreads, 1) attention_tile_kernel(const A
   load_tile(kbase, k_raw, k_s, 0);
   load_tile(vbase, v_raw, v_s, 0);
 
-  // value scales enter the weights relative to the chunk's largest one
-  float v_norm = static_cast<float>(1 << kWeightBits), v_unit = 1.0f / static_cast<float>(1 << kWeightBits);
-  if (kScaled) {
-    float top = 0.0f;
-#pragma unroll 4
-    for (int j = c0 + tid; j < c1; j += kTileThreads) {
-      const float s = fabsf(__ldg(p.vs + j));
-      bad |= !(s <= 3.402823466e38f);
-      top = fmaxf(top, s);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xFFFFFFFFu, top, o));
-    if (lane == 0) red[warp] = top;
-    __syncthreads();
-#pragma unroll
-    for (int w = 0; w < kTileThreads / 32; ++w) top = fmaxf(top, red[w]);
-    int e = static_cast<int>((__float_as_uint(top) >> 23) & 0xFFu) - 127;
-    e = max(kMinScaleExp, min(127, e));
-    if (top == 0.0f) e = 0;
-    v_norm = __uint_as_float(static_cast<uint32_t>(127 + kWeightBits - e) << 23);
-    v_unit = __uint_as_float(static_cast<uint32_t>(127 - kWeightBits + e) << 23);
-  }
   // queries, in base-2 exponents: each row scaled by a power of two to [2^13, 2^14), two binary16 terms.  A score's
   // factor is then its key's scale times a power of two.
   const float q_scale = kLog2e / sqrtf(static_cast<float>(D));
@@ -352,7 +337,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) attention_tile_kernel(const A
   if (kScaled) {
     const float s = load_scale(0);
     bad |= !(fabsf(s) <= 3.402823466e38f);
-    if (tid < 2 * kTileKeys) sc_s[tid] = tid < kTileKeys ? s : s * v_norm;
+    if (tid < 2 * kTileKeys) sc_s[tid] = s;
   }
   if (KV != kKvF16) {
     cp_async_wait<1>();
@@ -476,15 +461,35 @@ __global__ void __launch_bounds__(kTileThreads, 1) attention_tile_kernel(const A
         }
       }
       sum[0] += tile_sum[0], sum[1] += tile_sum[1];
+      float most[2] = {1.0f, 1.0f}, up[2], unit[2];
+      if (kScaled) {
+        most[0] = most[1] = 0.0f;
+#pragma unroll
+        for (int n = 0; n < kTileKeys / 8; ++n) {
+          const float2 f = *reinterpret_cast<const float2*>(vsc + n * 8 + (lane & 3) * 2);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            s[n][c] *= (c & 1) ? f.y : f.x;
+            most[c >> 1] = fmaxf(most[c >> 1], fabsf(s[n][c]));
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        if (kScaled) {
+          most[u] = fmaxf(most[u], __shfl_xor_sync(0xFFFFFFFFu, most[u], 1));
+          most[u] = fmaxf(most[u], __shfl_xor_sync(0xFFFFFFFFu, most[u], 2));
+        }
+        weight_unit(most[u], up[u], unit[u]);
+      }
       uint32_t ph[kTileKeys / 16][4], pl[kTileKeys / 16][4];
 #pragma unroll
       for (int kk = 0; kk < kTileKeys / 16; ++kk) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int n = 2 * kk + h;
-          const float2 f = kScaled ? *reinterpret_cast<const float2*>(vsc + n * 8 + (lane & 3) * 2) : make_float2(v_norm, v_norm);
-          split_half2(s[n][0] * f.x, s[n][1] * f.y, ph[kk][2 * h], pl[kk][2 * h]);
-          split_half2(s[n][2] * f.x, s[n][3] * f.y, ph[kk][2 * h + 1], pl[kk][2 * h + 1]);
+          split_half2(s[n][0] * up[0], s[n][1] * up[0], ph[kk][2 * h], pl[kk][2 * h]);
+          split_half2(s[n][2] * up[1], s[n][3] * up[1], ph[kk][2 * h + 1], pl[kk][2 * h + 1]);
         }
       }
 #pragma unroll
@@ -503,13 +508,16 @@ __global__ void __launch_bounds__(kTileThreads, 1) attention_tile_kernel(const A
             mma_f16(part[1], ph[kk], b[2], b[3]);
           }
 #pragma unroll
-          for (int c = 0; c < 4; ++c) o[2 * n][c] += part[0][c], o[2 * n + 1][c] += part[1][c];
+          for (int c = 0; c < 4; ++c) {
+            o[2 * n][c] = fmaf(part[0][c], unit[c >> 1], o[2 * n][c]);
+            o[2 * n + 1][c] = fmaf(part[1][c], unit[c >> 1], o[2 * n + 1][c]);
+          }
         }
       }
     }
     if (kScaled && tid < 2 * kTileKeys) {
       bad |= !(fabsf(next_scale) <= 3.402823466e38f);
-      sc_s[((t + 1) & 1) * 2 * kTileKeys + tid] = tid < kTileKeys ? next_scale : next_scale * v_norm;
+      sc_s[((t + 1) & 1) * 2 * kTileKeys + tid] = next_scale;
     }
     if (KV == kKvF16) {
       cp_async_wait<0>();
@@ -543,7 +551,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) attention_tile_kernel(const A
     const size_t head = static_cast<size_t>(kv) * group + g;
     if (tp.out != nullptr) {
       const size_t at = ((p.row_base + i) * p.heads + head) * D + (lane & 3) * 2;
-      const float f = v_unit / sum[u];
+      const float f = 1.0f / sum[u];
 #pragma unroll
       for (int n = 0; n < D / 8; ++n)
         *reinterpret_cast<float2*>(tp.out + at + n * 8) =
@@ -552,7 +560,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) attention_tile_kernel(const A
       const size_t part = (static_cast<size_t>(i) * p.heads + head) * chunk_stride + split;
 #pragma unroll
       for (int n = 0; n < D / 8; ++n)
-        *reinterpret_cast<float2*>(p.pacc + part * D + n * 8 + (lane & 3) * 2) = make_float2(o[n][2 * u] * v_unit, o[n][2 * u + 1] * v_unit);
+        *reinterpret_cast<float2*>(p.pacc + part * D + n * 8 + (lane & 3) * 2) = make_float2(o[n][2 * u], o[n][2 * u + 1]);
       if ((lane & 3) == 0) {
         p.pmax[part] = mx[u] == kNoKey ? kNullMax : mx[u] * kLn2;
         p.psum[part] = sum[u];
@@ -569,8 +577,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) attention_tile_kernel(const A
 // to MMA fragments in registers without shared memory, because the order of the elements along a contraction and of the
 // output rows is free: lane t of a key's four reads 16-byte pieces t, t + 4, ... of its row, and the queries are laid out in
 // that order; lane g of a value's eight reads the g-th eighth of its row.  The weights come out of the score MMA with keys
-// along g and are turned by movmatrix.  Two terms per query element and weight and exact cache elements as above; sixteen
-// keys' weights are normalised by their largest value scale.
+// along g and are turned by movmatrix.  Two terms per query element and weight and exact cache elements as above.
 constexpr int kFewWarps = 8, kFewKeys = 16, kFewCluster = 16;
 #ifndef FEWC
 #define FEWC 16
@@ -772,14 +779,7 @@ __global__ void __launch_bounds__(kFewWarps * 32, 1) attention_few_kernel(const 
     if (more) load_keys(base + kFewWarps * kFewKeys);
     bad |= !(fabsf(ks0) <= 3.402823466e38f) || !(fabsf(ks1) <= 3.402823466e38f) || !(fabsf(vs0) <= 3.402823466e38f) ||
            !(fabsf(vs1) <= 3.402823466e38f);
-    float vtop = fmaxf(fabsf(vs0), fabsf(vs1));
-#pragma unroll
-    for (int x = 4; x < 32; x <<= 1) vtop = fmaxf(vtop, __shfl_xor_sync(0xFFFFFFFFu, vtop, x));
-    int ev = static_cast<int>((__float_as_uint(vtop) >> 23) & 0xFFu) - 127;
-    ev = max(kMinScaleExp, min(127, ev));
-    if (vtop == 0.0f) ev = 0;
-    const float v_norm = __uint_as_float(static_cast<uint32_t>(127 + kWeightBits - ev) << 23);
-    const float v_unit = __uint_as_float(static_cast<uint32_t>(127 - kWeightBits + ev) << 23);
+    float unit[NT][2];
     uint32_t ph[NT][2], pl[NT][2];
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
@@ -805,9 +805,17 @@ __global__ void __launch_bounds__(kFewWarps * 32, 1) attention_few_kernel(const 
         for (int j = 0; j < D / 16; ++j)
           o[nt][j][0] *= corr[0], o[nt][j][1] *= corr[1], o[nt][j][2] *= corr[0], o[nt][j][3] *= corr[1];
       }
-      const float f0 = vs0 * v_norm, f1 = vs1 * v_norm;
-      split_half2(s[nt][0] * f0, s[nt][1] * f0, ph[nt][0], pl[nt][0]);
-      split_half2(s[nt][2] * f1, s[nt][3] * f1, ph[nt][1], pl[nt][1]);
+      float up[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        s[nt][u] *= vs0, s[nt][2 + u] *= vs1;
+        float most = fmaxf(fabsf(s[nt][u]), fabsf(s[nt][2 + u]));
+#pragma unroll
+        for (int x = 4; x < 32; x <<= 1) most = fmaxf(most, __shfl_xor_sync(0xFFFFFFFFu, most, x));
+        weight_unit(most, up[u], unit[nt][u]);
+      }
+      split_half2(s[nt][0] * up[0], s[nt][1] * up[1], ph[nt][0], pl[nt][0]);
+      split_half2(s[nt][2] * up[0], s[nt][3] * up[1], ph[nt][1], pl[nt][1]);
       ph[nt][0] = transpose_8x8(ph[nt][0]), ph[nt][1] = transpose_8x8(ph[nt][1]);
       pl[nt][0] = transpose_8x8(pl[nt][0]), pl[nt][1] = transpose_8x8(pl[nt][1]);
     }
@@ -852,7 +860,7 @@ __global__ void __launch_bounds__(kFewWarps * 32, 1) attention_few_kernel(const 
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
             float& sum_o = o[nt][w0 * kPer / 2 + x][c];
-            sum_o = fmaf(pt[x][nt][c], v_unit, sum_o);
+            sum_o = fmaf(pt[x][nt][c], unit[nt][c & 1], sum_o);
           }
     }
     if (more) load_values(base + kFewWarps * kFewKeys);

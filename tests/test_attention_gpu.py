@@ -313,6 +313,23 @@ SHAPES = [(22, 400, 24, 4, 256), (40, 4000, 16, 2, 128), (600, 64, 4, 2, 128), (
 
 
 @pytest.mark.parametrize("fmt", [2, 3, 4])
+@pytest.mark.parametrize("m,n,heads,kv_heads,head_dim", SHAPES)
+def test_value_scales_of_unlike_size(backend, oracle, fmt, m, n, heads, kv_heads, head_dim):
+    """Value scales over twelve decades, the largest on a key that only the last rows see, and a large one on a key of
+    negligible weight: every row is as exact as its own keys allow, whatever the other keys' scales are (the weights of a
+    row are split relative to that row's own largest contribution)."""
+    g = np.random.default_rng(100 + fmt + n)
+    q = g.standard_normal((m, heads * head_dim)).astype(np.float32)
+    k, v, ks, vs = make_cache(g, fmt, n, kv_heads * head_dim)
+    vs *= (10.0 ** g.uniform(-6, 6, n)).astype(np.float32)
+    q_base = max(0, n - m)
+    vs[n - max(1, min(m, n) // 2):] *= np.float32(1e9)
+    r = oracle.attention(fmt, q, k, v, m, n, heads, kv_heads, head_dim, q_base, 0, True, ks, vs)
+    y = device_attention(backend, fmt, q, k, v, ks, vs, m, n, heads, kv_heads, head_dim, q_base, 0, True)
+    assert near_each(y, r, head_dim)
+
+
+@pytest.mark.parametrize("fmt", [2, 3, 4])
 @pytest.mark.parametrize("exponent", [112, 103, -118])
 @pytest.mark.parametrize("m,n,heads,kv_heads,head_dim", SHAPES)
 def test_value_scales_at_the_ends_of_their_range(backend, oracle, fmt, exponent, m, n, heads, kv_heads, head_dim):
