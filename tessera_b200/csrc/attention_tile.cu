@@ -10,16 +10,22 @@
 // elements (FP8, int8, 4-bit, fp16) are exact in binary16, and a query element or a softmax weight enters as two
 // binary16 terms x = hi + lo of a value scaled by a power of two, 22 bits below the row's largest query element and
 // 2^-38 below the row's largest weight of a tile.  Scales of quantised rows multiply the score and the weight in fp32, the
-// latter before it is split: what a row does not see, or hardly weighs, takes nothing from it.  The MMA
-// cuts off what falls below its accumulator instead of rounding (chains over 4096 keys came out 4e-6 off), so two MMAs
-// of a score and eight of an output share an accumulator, the small terms first, before it is added in fp32: 3.8e-7
-// against 64 bits where the chunk kernel's fp32 sums have 3.0e-7 (longer chains 4.9e-7 at 6 % less time).
+// latter before it is split: what a row does not see, or hardly weighs, takes nothing from it.  The
+// MMA cuts off what falls below its accumulator instead of rounding (chains over 4096 keys came out 4e-6 off), and fp32 sums
+// round at every step, so: the small terms have accumulators of their own, where what is cut off does not count; the leading
+// terms of a score go through one MMA at a time, pairs of which are added to two sums, those of an output through four;
+// factor and maximum meet a score in one fused multiply-add; fp16 elements, whose products with a leading term are longer
+// than the accumulator, enter as their six leading bits and the rest.  Errors against 64 bits, the chunk kernel's in
+// brackets (512 rows, 4096 keys, 24 heads of 256; int8 2048 keys, 4-bit 300 rows): FP8 2.6e-7 (3.0e-7), int8 2.3e-7 (2.8e-7),
+// 4-bit 1.4e-7 (1.6e-7), fp16 2.16e-7 (2.19e-7).  With both terms in one accumulator, a single sum per score and a rounding
+// before the maximum is taken off it was 3.8e-7, 3.7e-7, 2.2e-7 and 3.1e-7, 6 % (fp16 45 %) faster.
 //
-// mma.sync rather than tcgen05: the 128 x 256 output accumulators have to be rescaled whenever a row's maximum
-// grows, which registers do in place and tensor memory only by a round trip; the two-term queries (128 KB) leave no
-// shared memory for the weights as a tcgen05 operand.
-// Bound: the tensor pipe, at the mma.sync rate: four MMAs where a plain product needs two.  512 rows over 4096 FP8 keys,
-// 24 heads of 256: 394 us against 4470 (123 TFLOP/s of the contract's 48 GFLOP, 246 of the MMAs').
+// Not built: the same on tcgen05, whose A operand can lie in tensor memory (weights without shared memory) and whose per-tile
+// sums would be added to fp32 registers as here.  Open there: the leading terms of a score keep their accuracy for one MMA of 16
+// elements, so every such product would be read back from tensor memory by itself.
+// Bound: the tensor pipe, at the mma.sync rate: four MMAs where a plain product needs two (fp16: six).  512 rows over 4096
+// keys, 24 heads of 256: FP8 423 us against the chunk kernel's 4470 (114 TFLOP/s of the contract's 48 GFLOP, 228 of the MMAs'),
+// fp16 589 us against 4615.  255 registers a thread, 16 to 84 bytes of them spilled.
 #include <cuda_fp16.h>
 
 #include <atomic>
@@ -32,7 +38,6 @@ namespace tsr {
 namespace {
 
 constexpr int kTileRows = 128, kTileKeys = 64, kTileThreads = 256;
-constexpr int kScoreChain = 1, kValueChain = 4;  // 16-wide k steps (of two MMAs) that share an accumulator
 constexpr int kWeightBits = 14;  // a row's largest weight (times its key's value scale) is stored in [2^14, 2^15)
 constexpr int kMinWeightExp = kWeightBits - 126;  // below, the power of two that takes it back would not be normal
 
@@ -80,6 +85,14 @@ __device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], u
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// The same from zero.
+__device__ __forceinline__ void mma_f16_first(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.0f));
+}
+__device__ __forceinline__ __half2 u32_half2(uint32_t v) { return *reinterpret_cast<const __half2*>(&v); }
 __device__ __forceinline__ uint32_t pack_half2(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
 // (x, y) as binary16 and what binary16 lost of them
 __device__ __forceinline__ void split_half2(float x, float y, uint32_t& hi, uint32_t& lo) {
@@ -88,7 +101,51 @@ __device__ __forceinline__ void split_half2(float x, float y, uint32_t& hi, uint
   hi = pack_half2(h);
   lo = pack_half2(__floats2half2_rn(x - f.x, y - f.y));
 }
-__device__ __forceinline__ __half2 u32_half2(uint32_t v) { return *reinterpret_cast<const __half2*>(&v); }
+
+// The same of the products x u and y v: one rounding, that of the second term.
+__device__ __forceinline__ void split_product2(float x, float y, float u, float v, uint32_t& hi, uint32_t& lo) {
+  const __half2 h = __floats2half2_rn(x * u, y * v);
+  const float2 f = __half22float2(h);
+  hi = pack_half2(h);
+  lo = pack_half2(__floats2half2_rn(fmaf(x, u, -f.x), fmaf(y, v, -f.y)));
+}
+// Leaves the six leading significant bits of two elements in place and returns the rest, both exact.
+__device__ __forceinline__ uint32_t split_elements(uint32_t& w) {
+  const uint32_t top = w & 0xFFE0FFE0u, rest = pack_half2(__hsub2(u32_half2(w), u32_half2(top)));
+  w = top;
+  return rest;
+}
+// sum + rest += x without a rounding at the sum's magnitude
+__device__ __forceinline__ void add_exact(float& sum, float& rest, float x) {
+  const float t = __fadd_rn(sum, x), z = __fsub_rn(t, sum);
+  rest = __fadd_rn(rest, __fadd_rn(__fsub_rn(sum, __fsub_rn(t, z)), __fsub_rn(x, z)));
+  sum = t;
+}
+// The two together; an infinite or NaN sum as it is (its rest is a NaN).
+__device__ __forceinline__ float with_rest(float sum, float rest) { return rest == rest ? sum + rest : sum; }
+// Pairwise sums (for their latency): with roundings on the way, and rounded once.
+template <int N>
+__device__ __forceinline__ float tree_sum(const float (&v)[N]) {
+  float s[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) s[i] = v[i];
+#pragma unroll
+  for (int half = N / 2; half > 0; half >>= 1)
+#pragma unroll
+    for (int i = 0; i < half; ++i) s[i] += s[i + half];
+  return s[0];
+}
+template <int N>
+__device__ __forceinline__ float exact_sum(const float (&v)[N]) {
+  float s[N], rest = 0.0f;
+#pragma unroll
+  for (int i = 0; i < N; ++i) s[i] = v[i];
+#pragma unroll
+  for (int half = N / 2; half > 0; half >>= 1)
+#pragma unroll
+    for (int i = 0; i < half; ++i) add_exact(s[i], rest, s[i + half]);
+  return with_rest(s[0], rest);
+}
 
 // A 16-byte piece of the cache as binary16 values; true when an element is not finite.
 __device__ __forceinline__ bool has_nonfinite_fp8(uint32_t w) { return (((w & 0x7F7F7F7Fu) + 0x01010101u) & 0x80808080u) != 0; }
@@ -134,6 +191,10 @@ __device__ __forceinline__ void weight_unit(float most, float& up, float& unit) 
   up = __uint_as_float(static_cast<uint32_t>(127 + kWeightBits - e) << 23);
   unit = __uint_as_float(static_cast<uint32_t>(127 - kWeightBits + e) << 23);
 }
+
+// exp2 of a score less the row's maximum.  The maximum is rounded and the difference is not, so x can lie above 0, by as much
+// as the scores' own error where they are beyond 2^24: a weight stays below 2 all the same.
+__device__ __forceinline__ float weight_of(float x) { return exp2f(fminf(x, 1.0f)); }
 
 // The keys [start, last] query row i sees.
 __device__ __forceinline__ void key_range(const AttnParams& p, int i, int& start, int& last) {
@@ -214,6 +275,7 @@ template <int KV, int D>
 __global__ void __launch_bounds__(kTileThreads, 1) attention_tile_kernel(const AttnTileParams tp) {
   using S = TileShape<KV, D>;
   constexpr bool kScaled = KV >= kKvFp8;
+  constexpr bool kLongElements = KV == kKvF16;  // eleven significant bits
   constexpr int kPitch = D * 2;  // bytes of a binary16 row
   extern __shared__ __align__(128) unsigned char smem[];
   unsigned char* const q_s = smem;  // [2 terms][128 rows][D]
@@ -284,8 +346,9 @@ __global__ void __launch_bounds__(kTileThreads, 1) attention_tile_kernel(const A
   load_tile(kbase, k_raw, k_s, 0);
   load_tile(vbase, v_raw, v_s, 0);
 
-  // queries, in base-2 exponents: each row scaled by a power of two to [2^13, 2^14), two binary16 terms.  A score's
-  // factor is then its key's scale times a power of two.
+  // queries: each row scaled by a power of two to [2^13, 2^14), two binary16 terms.  A score's factor (to a base-2 exponent)
+  // is then its key's scale times a power of two; without key scales it has room for 1 / sqrt(D) too, which rounds the
+  // elements otherwise.
   const float q_scale = kLog2e / sqrtf(static_cast<float>(D));
   constexpr int kRowsAtOnce = 4;  // loads in flight together
   for (int rr = 0; rr < 16; rr += kRowsAtOnce) {
@@ -305,7 +368,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) attention_tile_kernel(const A
 #pragma unroll
       for (int it = 0; it < D / 128; ++it) {
         float4& y = x[u][it];
-        y = make_float4(y.x * q_scale, y.y * q_scale, y.z * q_scale, y.w * q_scale);
+        if (kScaled) y = make_float4(y.x * q_scale, y.y * q_scale, y.z * q_scale, y.w * q_scale);
         bad |= !(fabsf(y.x) <= 3.402823466e38f) || !(fabsf(y.y) <= 3.402823466e38f) || !(fabsf(y.z) <= 3.402823466e38f) ||
                !(fabsf(y.w) <= 3.402823466e38f);
         top[u] = fmaxf(top[u], fmaxf(fmaxf(fabsf(y.x), fabsf(y.y)), fmaxf(fabsf(y.z), fabsf(y.w))));
@@ -322,7 +385,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) attention_tile_kernel(const A
       e = max(-110, min(114, e));
       if (top[u] == 0.0f) e = 0;
       const float up = __uint_as_float(static_cast<uint32_t>(127 - e) << 23);
-      if (lane == 0) row_f[r] = __uint_as_float(static_cast<uint32_t>(127 + e) << 23);
+      if (lane == 0) row_f[r] = __uint_as_float(static_cast<uint32_t>(127 + e) << 23) * (kScaled ? 1.0f : q_scale);
 #pragma unroll
       for (int it = 0; it < D / 128; ++it) {
         uint2 hi, lo;
@@ -366,7 +429,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) attention_tile_kernel(const A
   float o[D / 8][4];
 #pragma unroll
   for (int n = 0; n < D / 8; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.0f;
-  float mx[2] = {kNoKey, kNoKey}, sum[2] = {0.0f, 0.0f};
+  float mx[2] = {kNoKey, kNoKey}, sum[2] = {0.0f, 0.0f}, sum_rest[2] = {0.0f, 0.0f};
   const uint32_t q_addr = smem_addr(q_s) + (warp * 16 + (lane & 15)) * kPitch;
   const uint32_t k_addr = smem_addr(k_s) + ((lane & 7) + ((lane >> 4) << 3)) * kPitch;
   const uint32_t v_addr = smem_addr(v_s) + (lane & 15) * kPitch;
@@ -380,34 +443,46 @@ __global__ void __launch_bounds__(kTileThreads, 1) attention_tile_kernel(const A
 #pragma unroll
     for (int n = 0; n < kTileKeys / 8; ++n) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.0f;
     if (active) {
-#pragma unroll 4
-      for (int k4 = 0; k4 < D / 16 / kScoreChain; ++k4) {
-        float part[kTileKeys / 8][4];
 #pragma unroll
-        for (int n = 0; n < kTileKeys / 8; ++n) part[n][0] = part[n][1] = part[n][2] = part[n][3] = 0.0f;
+      for (int half = 0; half < 2; ++half) {  // 32 keys at a time: registers
+        constexpr int kN = kTileKeys / 16;
+        float low[kN][4] = {}, acc[2][kN][4] = {};
+#pragma unroll 1
+        for (int k4 = 0; k4 < D / 64; ++k4) {
+          float first[kN][4];
 #pragma unroll
-        for (int k1 = 0; k1 < kScoreChain; ++k1) {
-          const int kk = k4 * kScoreChain + k1;
-          uint32_t ah[4], al[4], b[kTileKeys / 16][4];
-          ldmatrix4(ah, q_addr + ((kk * 32) ^ q_x));
-          ldmatrix4(al, q_addr + S::kQBytes / 2 + ((kk * 32) ^ q_x));
+          for (int k1 = 0; k1 < 4; ++k1) {
+            const int kk = k4 * 4 + k1;
+            uint32_t ah[4], al[4], b[kN / 2][4];
+            ldmatrix4(ah, q_addr + ((kk * 32) ^ q_x));
+            ldmatrix4(al, q_addr + S::kQBytes / 2 + ((kk * 32) ^ q_x));
 #pragma unroll
-          for (int n = 0; n < kTileKeys / 16; ++n) ldmatrix4(b[n], k_addr + n * 16 * kPitch + ((kk * 32) ^ k_x));
+            for (int n = 0; n < kN / 2; ++n) ldmatrix4(b[n], k_addr + (half * 2 + n) * 16 * kPitch + ((kk * 32) ^ k_x));
+            float part[kN][4];
 #pragma unroll
-          for (int n = 0; n < kTileKeys / 16; ++n) {
-            mma_f16(part[2 * n], al, b[n][0], b[n][1]);
-            mma_f16(part[2 * n + 1], al, b[n][2], b[n][3]);
-          }
+            for (int n = 0; n < kN; ++n) mma_f16(low[n], al, b[n / 2][2 * (n & 1)], b[n / 2][2 * (n & 1) + 1]);
+            if constexpr (kLongElements) {
 #pragma unroll
-          for (int n = 0; n < kTileKeys / 16; ++n) {
-            mma_f16(part[2 * n], ah, b[n][0], b[n][1]);
-            mma_f16(part[2 * n + 1], ah, b[n][2], b[n][3]);
+              for (int n = 0; n < kN; ++n) {
+                const uint32_t r0 = split_elements(b[n / 2][2 * (n & 1)]), r1 = split_elements(b[n / 2][2 * (n & 1) + 1]);
+                mma_f16(low[n], ah, r0, r1);
+              }
+            }
+#pragma unroll
+            for (int n = 0; n < kN; ++n) mma_f16_first(part[n], ah, b[n / 2][2 * (n & 1)], b[n / 2][2 * (n & 1) + 1]);
+#pragma unroll
+            for (int n = 0; n < kN; ++n)
+#pragma unroll
+              for (int c = 0; c < 4; ++c) {
+                if (k1 % 2 == 0) first[n][c] = part[n][c];
+                else acc[k1 / 2][n][c] += first[n][c] + part[n][c];
+              }
           }
         }
 #pragma unroll
-        for (int n = 0; n < kTileKeys / 8; ++n)
+        for (int n = 0; n < kN; ++n)
 #pragma unroll
-          for (int c = 0; c < 4; ++c) s[n][c] += part[n][c];
+          for (int c = 0; c < 4; ++c) s[half * kN + n][c] = acc[0][n][c] + (acc[1][n][c] + low[n][c]);
       }
     }
     if (KV == kKvF16) cp_async_wait<0>();  // this tile's values (they were asked for after the tile before)
@@ -432,9 +507,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) attention_tile_kernel(const A
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           const int j = j0 + key + (c & 1);
-          const float v = s[n][c] * (rf[c >> 1] * ((c & 1) ? f.y : f.x));
-          s[n][c] = (j >= start[c >> 1] && j < stop[c >> 1]) ? v : kNoKey;
-          top[c >> 1] = fmaxf(top[c >> 1], s[n][c]);
+          if (j >= start[c >> 1] && j < stop[c >> 1]) top[c >> 1] = fmaxf(top[c >> 1], s[n][c] * (rf[c >> 1] * ((c & 1) ? f.y : f.x)));
+          else s[n][c] = kNoKey;
         }
       }
       float corr[2];
@@ -445,35 +519,28 @@ __global__ void __launch_bounds__(kTileThreads, 1) attention_tile_kernel(const A
         const float now = fmaxf(mx[u], top[u]);
         corr[u] = exp2f(mx[u] - now);  // 1 while the row has had no key (kNoKey - kNoKey)
         mx[u] = now;
-        sum[u] *= corr[u];
+        sum[u] *= corr[u], sum_rest[u] *= corr[u];
       }
       if (__any_sync(0xFFFFFFFFu, corr[0] != 1.0f || corr[1] != 1.0f)) {
 #pragma unroll
         for (int n = 0; n < D / 8; ++n) o[n][0] *= corr[0], o[n][1] *= corr[0], o[n][2] *= corr[1], o[n][3] *= corr[1];
       }
-      float tile_sum[2] = {0.0f, 0.0f};  // added to the running sum as one: fewer roundings at its magnitude
+      float tile_sum[2] = {0.0f, 0.0f}, most[2] = {kScaled ? 0.0f : 1.0f, kScaled ? 0.0f : 1.0f}, up[2], unit[2];
 #pragma unroll
       for (int n = 0; n < kTileKeys / 8; ++n) {
+        const int key = n * 8 + (lane & 3) * 2;
+        const float2 fk = kScaled ? *reinterpret_cast<const float2*>(ksc + key) : make_float2(1.0f, 1.0f);
+        const float2 fv = kScaled ? *reinterpret_cast<const float2*>(vsc + key) : make_float2(1.0f, 1.0f);
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          s[n][c] = s[n][c] == kNoKey ? 0.0f : exp2f(s[n][c] - mx[c >> 1]);
+          const float x = fmaf(s[n][c], rf[c >> 1] * ((c & 1) ? fk.y : fk.x), -mx[c >> 1]);
+          s[n][c] = s[n][c] == kNoKey ? 0.0f : weight_of(x);
           tile_sum[c >> 1] += s[n][c];
+          if (kScaled) most[c >> 1] = fmaxf(most[c >> 1], fabsf(s[n][c] * ((c & 1) ? fv.y : fv.x)));
         }
       }
-      sum[0] += tile_sum[0], sum[1] += tile_sum[1];
-      float most[2] = {1.0f, 1.0f}, up[2], unit[2];
-      if (kScaled) {
-        most[0] = most[1] = 0.0f;
-#pragma unroll
-        for (int n = 0; n < kTileKeys / 8; ++n) {
-          const float2 f = *reinterpret_cast<const float2*>(vsc + n * 8 + (lane & 3) * 2);
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            s[n][c] *= (c & 1) ? f.y : f.x;
-            most[c >> 1] = fmaxf(most[c >> 1], fabsf(s[n][c]));
-          }
-        }
-      }
+      add_exact(sum[0], sum_rest[0], tile_sum[0]);
+      add_exact(sum[1], sum_rest[1], tile_sum[1]);
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         if (kScaled) {
@@ -488,31 +555,37 @@ __global__ void __launch_bounds__(kTileThreads, 1) attention_tile_kernel(const A
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int n = 2 * kk + h;
-          split_half2(s[n][0] * up[0], s[n][1] * up[0], ph[kk][2 * h], pl[kk][2 * h]);
-          split_half2(s[n][2] * up[1], s[n][3] * up[1], ph[kk][2 * h + 1], pl[kk][2 * h + 1]);
+          const float2 fv = kScaled ? *reinterpret_cast<const float2*>(vsc + n * 8 + (lane & 3) * 2) : make_float2(1.0f, 1.0f);
+          split_product2(s[n][0] * up[0], s[n][1] * up[0], fv.x, fv.y, ph[kk][2 * h], pl[kk][2 * h]);
+          split_product2(s[n][2] * up[1], s[n][3] * up[1], fv.x, fv.y, ph[kk][2 * h + 1], pl[kk][2 * h + 1]);
         }
       }
 #pragma unroll
-      for (int k2 = 0; k2 < kTileKeys / 16 / kValueChain; ++k2) {
+      for (int n = 0; n < D / 16; ++n) {
+        float part[2][4], low[2][4];
 #pragma unroll
-        for (int n = 0; n < D / 16; ++n) {
-          float part[2][4] = {};
+        for (int kk = 0; kk < kTileKeys / 16; ++kk) {
+          uint32_t b[4];
+          ldmatrix4_trans(b, v_addr + kk * 16 * kPitch + ((n * 32) ^ v_x));
 #pragma unroll
-          for (int k1 = 0; k1 < kValueChain; ++k1) {
-            const int kk = k2 * kValueChain + k1;
-            uint32_t b[4];
-            ldmatrix4_trans(b, v_addr + kk * 16 * kPitch + ((n * 32) ^ v_x));
-            mma_f16(part[0], pl[kk], b[0], b[1]);
-            mma_f16(part[1], pl[kk], b[2], b[3]);
-            mma_f16(part[0], ph[kk], b[0], b[1]);
-            mma_f16(part[1], ph[kk], b[2], b[3]);
+          for (int h = 0; h < 2; ++h) {
+            if (kk == 0) mma_f16_first(low[h], pl[kk], b[2 * h], b[2 * h + 1]);
+            else mma_f16(low[h], pl[kk], b[2 * h], b[2 * h + 1]);
           }
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            o[2 * n][c] = fmaf(part[0][c], unit[c >> 1], o[2 * n][c]);
-            o[2 * n + 1][c] = fmaf(part[1][c], unit[c >> 1], o[2 * n + 1][c]);
+          for (int h = 0; h < 2; ++h) {
+            if constexpr (kLongElements) {
+              const uint32_t r0 = split_elements(b[2 * h]), r1 = split_elements(b[2 * h + 1]);
+              mma_f16(low[h], ph[kk], r0, r1);
+            }
+            if (kk == 0) mma_f16_first(part[h], ph[kk], b[2 * h], b[2 * h + 1]);
+            else mma_f16(part[h], ph[kk], b[2 * h], b[2 * h + 1]);
           }
         }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) o[2 * n + h][c] = fmaf(part[h][c] + low[h][c], unit[c >> 1], o[2 * n + h][c]);
       }
     }
     if (kScaled && tid < 2 * kTileKeys) {
@@ -543,6 +616,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) attention_tile_kernel(const A
   if (!active) return;
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
+    sum[u] = with_rest(sum[u], sum_rest[u]);
     sum[u] += __shfl_xor_sync(0xFFFFFFFFu, sum[u], 1);
     sum[u] += __shfl_xor_sync(0xFFFFFFFFu, sum[u], 2);
     const int r = r_lo + 8 * u;
@@ -617,6 +691,30 @@ __device__ __forceinline__ float ld_cluster(uint32_t addr) {
   float v;
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
   return v;
+}
+
+// One element of the result from `chunks` (<= N) CTAs' maximum, sum of weights and sum at these shared-memory addresses.
+template <int N>
+__device__ __forceinline__ float merged_chunks(int chunks, uint32_t top_at, uint32_t total_at, uint32_t acc_at) {
+  float tops[N], totals[N], accs[N], top = kNoKey;
+#pragma unroll
+  for (int c = 0; c < N; ++c) {
+    tops[c] = kNoKey, totals[c] = accs[c] = 0.0f;
+    if (c < chunks) {
+      tops[c] = ld_cluster(cluster_addr(top_at, c));
+      totals[c] = ld_cluster(cluster_addr(total_at, c));
+      accs[c] = ld_cluster(cluster_addr(acc_at, c));
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < N; ++c) top = fmaxf(top, tops[c]);
+#pragma unroll
+  for (int c = 0; c < N; ++c)
+    if (c < chunks) {
+      const float w = exp2f(tops[c] - top);
+      accs[c] *= w, totals[c] *= w;
+    }
+  return exact_sum(accs) / exact_sum(totals);
 }
 
 // grid: (kv_heads * splits, row tiles) in clusters of (splits, 1)
@@ -750,7 +848,7 @@ __global__ void __launch_bounds__(kFewWarps * 32, 1) attention_few_kernel(const 
 #pragma unroll
     for (int w0 = 0; w0 < 4 * S::kKeyPieces; w0 += kGroup / kWordSteps) {
       uint32_t b[2][kGroup / kWordSteps][2 * kWordSteps];
-      float pt[kGroup][NT][4] = {};
+      float pt[kGroup][NT][4];
 #pragma unroll
       for (int x = 0; x < kGroup / kWordSteps; ++x) {
         bad |= expand_word<KV>(kraw[0][(w0 + x) / 4][(w0 + x) % 4], b[0][x]);
@@ -765,15 +863,14 @@ __global__ void __launch_bounds__(kFewWarps * 32, 1) attention_few_kernel(const 
 #pragma unroll
           for (int nt = 0; nt < NT; ++nt) {
             const uint2 f = *reinterpret_cast<const uint2*>(q_s + (((w0 * kWordSteps + x) * NT + nt) * 64 + lo * 32 + lane) * 2);
-            mma_f16(pt[x][nt], a, f.x, f.y);
+            if (lo) mma_f16_first(pt[x][nt], a, f.x, f.y);
+            else mma_f16(pt[x][nt], a, f.x, f.y);
           }
         }
 #pragma unroll
-      for (int x = 0; x < kGroup; ++x)
+      for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-          for (int c = 0; c < 4; ++c) s[nt][c] += pt[x][nt][c];
+        for (int c = 0; c < 4; ++c) s[nt][c] += (pt[0][nt][c] + pt[1][nt][c]) + (pt[2][nt][c] + pt[3][nt][c]);
     }
     const float ks0 = ksc[0], ks1 = ksc[1], vs0 = vsc[0], vs1 = vsc[1];
     if (more) load_keys(base + kFewWarps * kFewKeys);
@@ -787,17 +884,16 @@ __global__ void __launch_bounds__(kFewWarps * 32, 1) attention_few_kernel(const 
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         const int j = base + g;
-        const float x0 = s[nt][u] * (rf[nt][u] * ks0), x1 = s[nt][2 + u] * (rf[nt][u] * ks1);
-        s[nt][u] = (j >= start[nt][u] && j < stop[nt][u]) ? x0 : kNoKey;
-        s[nt][2 + u] = (j + 8 >= start[nt][u] && j + 8 < stop[nt][u]) ? x1 : kNoKey;
-        float top = fmaxf(s[nt][u], s[nt][2 + u]);
+        const float f0 = rf[nt][u] * ks0, f1 = rf[nt][u] * ks1;
+        const bool in0 = j >= start[nt][u] && j < stop[nt][u], in1 = j + 8 >= start[nt][u] && j + 8 < stop[nt][u];
+        float top = fmaxf(in0 ? s[nt][u] * f0 : kNoKey, in1 ? s[nt][2 + u] * f1 : kNoKey);
 #pragma unroll
         for (int x = 4; x < 32; x <<= 1) top = fmaxf(top, __shfl_xor_sync(0xFFFFFFFFu, top, x));
         const float now = fmaxf(mx[nt][u], top);
         corr[u] = exp2f(mx[nt][u] - now);
         mx[nt][u] = now;
-        s[nt][u] = s[nt][u] == kNoKey ? 0.0f : exp2f(s[nt][u] - now);
-        s[nt][2 + u] = s[nt][2 + u] == kNoKey ? 0.0f : exp2f(s[nt][2 + u] - now);
+        s[nt][u] = in0 ? weight_of(fmaf(s[nt][u], f0, -now)) : 0.0f;
+        s[nt][2 + u] = in1 ? weight_of(fmaf(s[nt][2 + u], f1, -now)) : 0.0f;
         sum[nt][u] = fmaf(sum[nt][u], corr[u], s[nt][u] + s[nt][2 + u]);
       }
       if (__any_sync(0xFFFFFFFFu, corr[0] != 1.0f || corr[1] != 1.0f)) {
@@ -808,14 +904,13 @@ __global__ void __launch_bounds__(kFewWarps * 32, 1) attention_few_kernel(const 
       float up[2];
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
-        s[nt][u] *= vs0, s[nt][2 + u] *= vs1;
-        float most = fmaxf(fabsf(s[nt][u]), fabsf(s[nt][2 + u]));
+        float most = fmaxf(fabsf(s[nt][u] * vs0), fabsf(s[nt][2 + u] * vs1));
 #pragma unroll
         for (int x = 4; x < 32; x <<= 1) most = fmaxf(most, __shfl_xor_sync(0xFFFFFFFFu, most, x));
         weight_unit(most, up[u], unit[nt][u]);
       }
-      split_half2(s[nt][0] * up[0], s[nt][1] * up[1], ph[nt][0], pl[nt][0]);
-      split_half2(s[nt][2] * up[0], s[nt][3] * up[1], ph[nt][1], pl[nt][1]);
+      split_product2(s[nt][0] * up[0], s[nt][1] * up[1], vs0, vs0, ph[nt][0], pl[nt][0]);
+      split_product2(s[nt][2] * up[0], s[nt][3] * up[1], vs1, vs1, ph[nt][1], pl[nt][1]);
       ph[nt][0] = transpose_8x8(ph[nt][0]), ph[nt][1] = transpose_8x8(ph[nt][1]);
       pl[nt][0] = transpose_8x8(pl[nt][0]), pl[nt][1] = transpose_8x8(pl[nt][1]);
     }
@@ -841,7 +936,7 @@ __global__ void __launch_bounds__(kFewWarps * 32, 1) attention_few_kernel(const 
             for (int x4 = 0; x4 < 4; ++x4) dst[2 * x4] = x[x4], dst[2 * x4 + 1] = y[x4];
           }
         }
-      float pt[kGroup][NT][4] = {};
+      float pt[kGroup][NT][4];
 #pragma unroll
       for (int lo = 1; lo >= 0; --lo)
 #pragma unroll
@@ -849,7 +944,7 @@ __global__ void __launch_bounds__(kFewWarps * 32, 1) attention_few_kernel(const 
           const uint32_t a[4] = {b[0][2 * x], b[0][2 * x + 1], b[1][2 * x], b[1][2 * x + 1]};
 #pragma unroll
           for (int nt = 0; nt < NT; ++nt) {
-            if (lo) mma_f16(pt[x][nt], a, pl[nt][0], pl[nt][1]);
+            if (lo) mma_f16_first(pt[x][nt], a, pl[nt][0], pl[nt][1]);
             else mma_f16(pt[x][nt], a, ph[nt][0], ph[nt][1]);
           }
         }
@@ -868,7 +963,7 @@ __global__ void __launch_bounds__(kFewWarps * 32, 1) attention_few_kernel(const 
   if (__syncthreads_or(bad)) {
     scalar_rows<KV, D>(p, kv, group, row0, rows, c0, c1, split, warp, kFewWarps, nullptr, nullptr, acc_s, top_s, total_s);
   } else {
-    // the warps meet: the CTA's max per row, every warp's share rescaled to it, summed in warp order
+    // the warps meet: the CTA's max per row, every warp's share rescaled to it
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -896,49 +991,35 @@ __global__ void __launch_bounds__(kFewWarps * 32, 1) attention_few_kernel(const 
     for (int x = tid; x < rows * D; x += kFewWarps * 32) {
       const int r = x / D, d = x - r * D;
       const float* src = part + r * S::kPitch + d / (D / 8) * S::kEighth + d % (D / 8);
-      float total = 0.0f;
+      float v[kFewWarps];
 #pragma unroll
-      for (int w = 0; w < kFewWarps; ++w) total += src[w * kRows * S::kPitch];
-      acc_s[x] = total;
+      for (int w = 0; w < kFewWarps; ++w) v[w] = src[w * kRows * S::kPitch];
+      acc_s[x] = tree_sum(v);
     }
     if (tid < rows) {
-      float top = wmax[tid], total = 0.0f;
+      float top = wmax[tid], v[kFewWarps];
 #pragma unroll
       for (int w = 1; w < kFewWarps; ++w) top = fmaxf(top, wmax[w * kRows + tid]);
 #pragma unroll
-      for (int w = 0; w < kFewWarps; ++w) total += wsum[w * kRows + tid];
-      top_s[tid] = top, total_s[tid] = total;
+      for (int w = 0; w < kFewWarps; ++w) v[w] = wsum[w * kRows + tid];
+      top_s[tid] = top, total_s[tid] = tree_sum(v);
     }
   }
   // the chunks meet: CTA `split` merges its share of the elements, all CTAs' values in flight
   cluster_sync();
   const int share = (rows * D + p.splits - 1) / p.splits;
-  for (int x = split * share + tid; x < min(rows * D, (split + 1) * share); x += kFewWarps * 32) {
+  const int begin_x = split * share + tid, end_x = min(rows * D, (split + 1) * share);
+  for (int x = begin_x; x < end_x; x += kFewWarps * 32) {
     const int r = x / D, d = x - r * D, i = (row0 + r) / group, hd = (row0 + r) - i * group;
-    float tops[kFewCluster], totals[kFewCluster], accs[kFewCluster], top = kNoKey, num = 0.0f, den = 0.0f;
-#pragma unroll
-    for (int c = 0; c < kFewCluster; ++c)
-      if (c < p.splits) {
-        tops[c] = ld_cluster(cluster_addr(smem_addr(top_s + r), c));
-        totals[c] = ld_cluster(cluster_addr(smem_addr(total_s + r), c));
-        accs[c] = ld_cluster(cluster_addr(smem_addr(acc_s + x), c));
-      }
-#pragma unroll
-    for (int c = 0; c < kFewCluster; ++c)
-      if (c < p.splits) top = fmaxf(top, tops[c]);
-#pragma unroll
-    for (int c = 0; c < kFewCluster; ++c)
-      if (c < p.splits) {
-        const float w = exp2f(tops[c] - top);
-        num = fmaf(w, accs[c], num), den = fmaf(w, totals[c], den);
-      }
+    const uint32_t top_at = smem_addr(top_s + r), total_at = smem_addr(total_s + r), acc_at = smem_addr(acc_s + x);
+    const float v = p.splits <= 4 ? merged_chunks<4>(p.splits, top_at, total_at, acc_at) : merged_chunks<kFewCluster>(p.splits, top_at, total_at, acc_at);
     const size_t at = ((p.row_base + i) * p.heads + static_cast<size_t>(kv) * group + hd) * D + d;
-    out[at] = gated(num / den, gate, at);
+    out[at] = gated(v, gate, at);
   }
   cluster_sync();  // the others may still read this CTA's sums
 }
 
-// The chunks of a (row, head): a thread per four elements, chunks in order (attention_combine's arithmetic; that
+// The chunks of a (row, head): a thread per four elements, chunks in order (that of attention_combine; its
 // kernel spends a CTA on 64 elements of one row, which costs more than the reads once there are thousands of rows).
 __global__ void __launch_bounds__(256)
 attention_merge_kernel(const float* __restrict__ pacc, const float* __restrict__ pmax, const float* __restrict__ psum,
@@ -947,19 +1028,22 @@ attention_merge_kernel(const float* __restrict__ pacc, const float* __restrict__
   const size_t t = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t >= total) return;
   const size_t row = t / dim4, e = t - row * dim4, base = row * splits;
-  float top = kNullMax, den = 0.0f;
+  float top = kNullMax, den = 0.0f, den_rest = 0.0f, num[4] = {}, rest[4] = {};
   for (int s = 0; s < splits; ++s) top = fmaxf(top, pmax[base + s]);
-  float4 num = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll 4
   for (int s = 0; s < splits; ++s) {
     const float w = expf(pmax[base + s] - top);
     const float4 x = reinterpret_cast<const float4*>(pacc)[(base + s) * dim4 + e];
-    den = fmaf(w, psum[base + s], den);
-    num = make_float4(fmaf(w, x.x, num.x), fmaf(w, x.y, num.y), fmaf(w, x.z, num.z), fmaf(w, x.w, num.w));
+    add_exact(den, den_rest, w * psum[base + s]);
+    add_exact(num[0], rest[0], w * x.x), add_exact(num[1], rest[1], w * x.y);
+    add_exact(num[2], rest[2], w * x.z), add_exact(num[3], rest[3], w * x.w);
   }
+  den = with_rest(den, den_rest);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) num[c] = with_rest(num[c], rest[c]);
   const size_t at = (out_base + t) * 4;
-  *reinterpret_cast<float4*>(out + at) = make_float4(gated(num.x / den, gate, at), gated(num.y / den, gate, at + 1),
-                                                     gated(num.z / den, gate, at + 2), gated(num.w / den, gate, at + 3));
+  *reinterpret_cast<float4*>(out + at) = make_float4(gated(num[0] / den, gate, at), gated(num[1] / den, gate, at + 1),
+                                                     gated(num[2] / den, gate, at + 2), gated(num[3] / den, gate, at + 3));
 }
 
 template <int KV, int D>

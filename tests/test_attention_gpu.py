@@ -6,6 +6,7 @@ import os
 
 import numpy as np
 import pytest
+import torch
 
 from tessera_b200 import capi
 from tessera_b200.backend import KernelLaunch
@@ -345,3 +346,62 @@ def test_value_scales_at_the_ends_of_their_range(backend, oracle, fmt, exponent,
     y = device_attention(backend, fmt, q, k, v, ks, vs * factor, m, n, heads, kv_heads, head_dim, q_base, 0, True)
     assert np.isfinite(y).all()
     assert near_each(y / factor, r, head_dim)
+
+
+def decoded64(fmt, cache, scale, n):
+    """A cache in 64 bits."""
+    if fmt == 1:
+        return cache.view(np.float16).reshape(n, -1).astype(np.float64)
+    if fmt == 2:
+        x = cache.view(np.int8).astype(np.float64)
+    elif fmt == 3:
+        x = np.stack([cache & 15, cache >> 4], 2).reshape(n, -1).astype(np.float64)
+        x = np.where(x >= 8, x - 16, x)
+    else:
+        mag, man = (cache >> 3) & 15, (cache & 7).astype(np.float64)
+        x = np.where(mag == 0, man / 8 * 2.0 ** -6, (1 + man / 8) * 2.0 ** (mag.astype(np.float64) - 7))
+        x = np.where(cache & 0x80, -x, x)
+    return x.reshape(n, -1) * scale.astype(np.float64)[:, None]
+
+
+def attention64(q, k, v, heads, kv_heads, head_dim, q_base):
+    m, n = q.shape[0], k.shape[0]
+    hidden = np.arange(n)[None] > q_base + np.arange(m)[:, None]
+    q, k, v = (x.reshape(-1, h, head_dim).astype(np.float64) for x, h in ((q, heads), (k, kv_heads), (v, kv_heads)))
+    out = np.empty_like(q)
+    for h in range(heads):
+        s = q[:, h] @ k[:, h * kv_heads // heads].T / np.sqrt(head_dim)
+        s[hidden] = -np.inf
+        w = np.exp(s - s.max(1, keepdims=True))
+        out[:, h] = (w / w.sum(1, keepdims=True)) @ v[:, h * kv_heads // heads]
+    return out.reshape(m, -1)
+
+
+@pytest.mark.parametrize("fmt", [1, 2, 3, 4])
+@pytest.mark.parametrize("m,n,heads,kv_heads,head_dim,draws", [(96, 2048, 16, 2, 256, 2), (160, 1500, 8, 2, 128, 3), (1, 4096, 24, 4, 256, 12),
+                                                               (3, 2000, 16, 2, 128, 12)])
+def test_as_close_to_64_bits_as_fp32_sums(backend, fmt, m, n, heads, kv_heads, head_dim, draws):
+    """The tensor-pipe kernels against attention_*_split and attention_combine, whose products and sums are fp32 throughout:
+    the error (2-norm, over all draws) is no larger, on keys and values of unit size.  2 %: the spread between draws."""
+    mine = chunks = 0.0
+    for seed in range(draws):
+        g = np.random.default_rng(1000 * fmt + seed)
+        q = g.standard_normal((m, heads * head_dim)).astype(np.float32)
+        k, v, ks, vs = make_cache(g, fmt, n, kv_heads * head_dim)
+        if fmt == 4:
+            k, v = (torch.from_numpy(np.clip(g.standard_normal(x.shape).astype(np.float32) * 100, -448, 448)).to(torch.float8_e4m3fn).view(torch.uint8).numpy() for x in (k, v))
+        ks, vs = (g.uniform(0.5, 1.5, n).astype(np.float32) / np.float32({1: 1, 2: 74, 3: 4.6, 4: 100}[fmt]) for _ in range(2))
+        want = attention64(q, decoded64(fmt, k, ks, n), decoded64(fmt, v, vs, n), heads, kv_heads, head_dim, n - m)
+        y = device_attention(backend, fmt, q, k, v, ks, vs, m, n, heads, kv_heads, head_dim, n - m, 0, True)
+        split = min(64, n // 64)
+        bufs = [backend.upload(x) for x in ((q, k, v) if fmt == 1 else (q, k, v, ks, vs))]
+        parts = [backend.AllocateBuffer(m * heads * split * c * 4) for c in (head_dim, 1, 1)]
+        out = backend.AllocateBuffer(q.nbytes)
+        run(backend, "attention_split" if fmt == 1 else QUANT_ID[fmt] + "_split", bufs + parts,
+            [m, n, heads, kv_heads, head_dim, n - m, 0] + ([1, 1] if fmt == 1 else [QUANT_KIND[fmt]]) + [split])
+        run(backend, "attention_combine", parts + [out], [m, heads, head_dim, split])
+        x = backend.download(out, np.float32, q.size).reshape(q.shape)
+        mine += float(np.sum((y - want) ** 2) / np.sum(want ** 2))
+        chunks += float(np.sum((x - want) ** 2) / np.sum(want ** 2))
+    print("error %.3e, fp32 sums %.3e" % ((mine / draws) ** 0.5, (chunks / draws) ** 0.5))
+    assert mine <= 1.04 * chunks      # (1.02 ** 2)
