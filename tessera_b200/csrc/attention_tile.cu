@@ -31,13 +31,14 @@
 #include <atomic>
 
 #include "attention.cuh"
+#include "attention_plan.h"
 #include "codec.cuh"
 #include "launch.h"
 
 namespace tsr {
 namespace {
 
-constexpr int kTileRows = 128, kTileKeys = 64, kTileThreads = 256;
+constexpr int kTileThreads = 256;
 constexpr int kWeightBits = 14;  // a row's largest weight (times its key's value scale) is stored in [2^14, 2^15)
 constexpr int kMinWeightExp = kWeightBits - 126;  // below, the power of two that takes it back would not be normal
 
@@ -1148,11 +1149,7 @@ int attention_few(int kvkind, AttnParams p, float* out, const float* gate, cudaS
 int attention_tile(int kvkind, AttnParams p, float* out, const float* gate, cudaStream_t st) {
   const int group = p.heads / p.kv_heads;
   const long rows = static_cast<long>(p.m) * group;
-  // keys a row tile walks over: the window of its first row to the position of its last
-  long span = p.n;
-  if (p.causal && p.window != 0) span = span < p.window + kTileRows / group + 1 ? span : p.window + kTileRows / group + 1;
-  if (p.causal && p.q_base + static_cast<unsigned long long>(p.m) < static_cast<unsigned long long>(span))
-    span = static_cast<long>(p.q_base) + p.m;
+  const long span = static_cast<long>(tile_span(p.m, p.n, p.q_base, p.window, p.causal != 0, group));
   // Below a few rows a CTA's 128-row tile is mostly empty, and a short call is over before the tile's start has paid
   // off: measured (FP8, chunk kernel -> here) 8 rows x 200 keys 18 -> 20 us, 16 x 300 22.8 -> 23.8, 8 x 1024 28.9 -> 22.8,
   // 4 x 4096 45 -> 30, 16 x 4096 150 -> 36 (24 heads over 4 of 256); 2 rows x 4096 29 -> 29.
