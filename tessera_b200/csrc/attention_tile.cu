@@ -653,16 +653,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) attention_tile_kernel(const A
 // output rows is free: lane t of a key's four reads 16-byte pieces t, t + 4, ... of its row, and the queries are laid out in
 // that order; lane g of a value's eight reads the g-th eighth of its row.  The weights come out of the score MMA with keys
 // along g and are turned by movmatrix.  Two terms per query element and weight and exact cache elements as above.
-constexpr int kFewWarps = 8, kFewKeys = 16, kFewCluster = 16;
-#ifndef FEWC
-#define FEWC 16
-#endif
-#ifndef FEWG
-#define FEWG 4
-#endif
-#ifndef FEWW
-#define FEWW 64
-#endif
+constexpr int kFewWarps = 8, kFewKeys = 16;  // a warp's keys at a time
 
 template <int KV, int D, int NT>
 struct FewShape {
@@ -725,7 +716,8 @@ __global__ void __launch_bounds__(kFewWarps * 32, 1) attention_few_kernel(const 
   static_assert(kv_bits<KV>() <= 8, "formats with a scale per row");
   constexpr int kWordSteps = kv_bits<KV>() == 8 ? 1 : 2;  // k steps a 32-bit word of a key feeds
   constexpr int kPer = 32 / kv_bits<KV>();                // elements of a word
-  constexpr int kGroup = FEWG;  // MMA pairs in flight: the second of a pair waits for the first
+  constexpr int kGroup = 4;  // MMA pairs in flight: the second of a pair waits for the first
+  static_assert(4 * S::kKeyPieces % (kGroup / kWordSteps) == 0 && S::kValueWords % (2 * kGroup / kPer) == 0, "whole groups");
   constexpr int kRows = S::kRows;
   extern __shared__ __align__(128) unsigned char smem[];
   uint32_t* const q_s = reinterpret_cast<uint32_t*>(smem);                 // [D / 16][NT][hi, lo][32 lanes][2]
@@ -1136,9 +1128,8 @@ int attention_few(int kvkind, AttnParams p, float* out, const float* gate, cudaS
   const long span = p.causal && p.window != 0 && p.window < p.n ? p.window : p.n;
   if (kvkind < kKvFp8 || !aligned16(p.q) || !aligned16(p.k) || !aligned16(p.v) || !writes_apart(kvkind, p, out, gate))
     return kUnsupportedFeature;
-  // a warp's sixteen keys in each CTA before another CTA joins
   p.splits = 1;
-  while (p.splits < FEWC && p.splits * FEWW < span) p.splits *= 2;
+  while (p.splits < kFewCluster && p.splits * kFewKeysPerCta < span) p.splits *= 2;
   switch (kvkind) {
     case kKvFp8: return launch_few<kKvFp8>(p, group, out, gate, st);
     case kKvInt8: return launch_few<kKvInt8>(p, group, out, gate, st);
