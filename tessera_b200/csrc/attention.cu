@@ -407,8 +407,8 @@ int run_attention(int kvkind, const float* q, const void* k, const void* v, cons
   AttnParams p;
   if (int rc = check_attention(kvkind, q, k, v, ks, vs, m, n, heads, kv_heads, head_dim, q_base, row_base, window, causal, 1, &p))
     return rc;
-  int rc = attention_tile(kvkind, p, out, gate, st);
-  if (rc == kUnsupportedFeature) rc = attention_few(kvkind, p, out, gate, st);
+  int rc = attention_few(kvkind, p, out, gate, st);
+  if (rc == kUnsupportedFeature) rc = attention_tile(kvkind, p, out, gate, st);
   if (rc != kUnsupportedFeature) return rc;
   // as many chunks as keep a CTA busy with kAttnMinKeys keys, counted on the longest row's range
   const uint64_t span = window != 0 && window < n ? window : n;

@@ -40,7 +40,8 @@ struct AttnParams {
 // 16-bit and narrower caches, out = attention [* sigmoid(gate)].  kUnsupportedFeature: not one of its shapes.
 int attention_tile(int kvkind, AttnParams p, float* out, const float* gate, cudaStream_t st);
 
-// The same of a few rows over an FP8, int8 or 4-bit cache.
+// The same of few (row, head) pairs or keys over an FP8, int8 or 4-bit cache: asked first, kUnsupportedFeature where row
+// tiles are the better choice too.
 int attention_few(int kvkind, AttnParams p, float* out, const float* gate, cudaStream_t st);
 
 }  // namespace tsr

@@ -644,15 +644,19 @@ __global__ void __launch_bounds__(kTileThreads, 1) attention_tile_kernel(const A
   }
 }
 
-// ---- few rows (a decoded token, two or three drafted ones) ----
+// ---- few rows (a decoded token, drafted ones, a short prompt) ----
 // The chunk kernel of attention.cu is bound by its instructions (about 1000 for four keys of a warp), and its chunks meet
-// in a second launch.  Here a cluster of up to sixteen CTAs takes one kv head and 8 NT (row, head) pairs over the whole key
-// range: a CTA a chunk, a warp sixteen keys at a time, and the chunks meet through distributed shared memory.
+// in a second launch; a row tile is mostly padding.  Here a cluster of up to sixteen CTAs takes one kv head and 8 NT
+// (row, head) pairs over the whole key range: a CTA a chunk, a warp sixteen keys at a time, and the chunks meet through
+// distributed shared memory.  More pairs are more clusters, as long as they all run at a time (few_ctas, few_rows_win).
 // The products are S^T = K Q^T and O^T = V^T P^T, so that eight rows fill an MMA.  Keys and values go from global memory
 // to MMA fragments in registers without shared memory, because the order of the elements along a contraction and of the
 // output rows is free: lane t of a key's four reads 16-byte pieces t, t + 4, ... of its row, and the queries are laid out in
 // that order; lane g of a value's eight reads the g-th eighth of its row.  The weights come out of the score MMA with keys
-// along g and are turned by movmatrix.  Two terms per query element and weight and exact cache elements as above.
+// along g and are turned by movmatrix.  Two terms per query element and weight and exact cache elements as above; the MMAs
+// of four steps are added pairwise and the cluster's chunks without roundings.  One row of 24 heads over 4 of 256 and 4096 FP8
+// keys 11.7 us (chunk kernel 15.2) at 2.2e-7 against 64 bits (2.9e-7).  Bound: latency (64 CTAs, two trips a warp) and the
+// registers: 179 to 255 a thread, and with sixteen rows of 256 up to 432 bytes spilled.
 constexpr int kFewWarps = 8, kFewKeys = 16;  // a warp's keys at a time
 
 template <int KV, int D, int NT>
@@ -1054,58 +1058,73 @@ int launch_tile_d(const AttnTileParams& tp, cudaStream_t st) {
   return tp.a.head_dim == 256 ? launch_tile<KV, 256>(tp, st) : launch_tile<KV, 128>(tp, st);
 }
 
-// kUnsupportedFeature where the device does not take clusters of that size (a partitioned GPU).
+bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
 template <int KV, int D, int NT>
-int launch_few_nt(AttnParams p, int group, float* out, const float* gate, cudaStream_t st) {
+cudaLaunchConfig_t few_config(cudaLaunchAttribute* cluster, int ctas, dim3 grid, cudaStream_t st) {
+  cluster->id = cudaLaunchAttributeClusterDimension;
+  cluster->val.clusterDim.x = static_cast<unsigned>(ctas);
+  cluster->val.clusterDim.y = cluster->val.clusterDim.z = 1;
+  cudaLaunchConfig_t config{};
+  config.gridDim = grid;
+  config.blockDim = dim3(kFewWarps * 32);
+  config.dynamicSmemBytes = FewShape<KV, D, NT>::kSmem;
+  config.stream = st;
+  config.attrs = cluster;
+  config.numAttrs = 1;
+  return config;
+}
+
+// Clusters of `ctas` CTAs (a power of two) that the device runs at a time: a cluster lies within a GPC, so a B200 holds few
+// of sixteen, more than twice as many of eight.  0 where it takes none of that size (a partitioned GPU).
+template <int KV, int D, int NT>
+int few_resident(int dev, int ctas) {
+  static std::atomic<int> known[64][5];  // the number plus one; 0: not asked
+  int log = 0;
+  while ((1 << log) < ctas) ++log;
+  if (int v = known[dev][log].load(std::memory_order_relaxed)) return v - 1;
+  const auto kernel = &attention_few_kernel<KV, D, NT>;
+  cudaLaunchAttribute cluster;
+  const cudaLaunchConfig_t config = few_config<KV, D, NT>(&cluster, ctas, dim3(static_cast<unsigned>(ctas)), nullptr);
+  int clusters = 0;
+  if ((ctas > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
+      cudaOccupancyMaxActiveClusters(&clusters, kernel, &config) != cudaSuccess) {
+    cudaGetLastError();
+    clusters = 0;
+  }
+  known[dev][log].store(clusters + 1, std::memory_order_relaxed);
+  return clusters;
+}
+
+template <int KV, int D, int NT>
+int launch_few_nt(AttnParams p, long span, int group, float* out, const float* gate, cudaStream_t st) {
   using S = FewShape<KV, D, NT>;
   const auto kernel = &attention_few_kernel<KV, D, NT>;
   if (int rc = allow_dynamic_smem(reinterpret_cast<const void*>(kernel), S::kSmem)) return rc;
-  static std::atomic<int> resident[64];  // per device: clusters of sixteen that run at a time, plus one; 0 not asked
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return kDeviceError;
-  cudaLaunchConfig_t config{};
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  config.blockDim = dim3(kFewWarps * 32);
-  config.dynamicSmemBytes = S::kSmem;
-  config.stream = st;
-  config.attrs = attr;
-  config.numAttrs = 1;
-  if (resident[dev].load(std::memory_order_relaxed) == 0) {
-    int clusters = 0;
-    attr[0].val.clusterDim.x = kFewCluster;
-    config.gridDim = dim3(kFewCluster);
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&clusters, kernel, &config) != cudaSuccess) {
-      cudaGetLastError();
-      clusters = 0;
-    }
-    resident[dev].store(clusters + 1, std::memory_order_relaxed);
-  }
-  const int fit = resident[dev].load(std::memory_order_relaxed) - 1, row_tiles = (p.m * group + S::kRows - 1) / S::kRows;
-  if (fit == 0) return kUnsupportedFeature;
-  // A GPU holds few clusters of sixteen (the SMs of one GPC each), twice as many of eight and a rest: a second wave costs
-  // more than twice the keys per CTA.  2 rows x 4096 keys, 32 heads over 8 of 128: 303 us a pass in sixteens, 201 in eights.
-  if (p.splits == kFewCluster && p.kv_heads * row_tiles > fit) p.splits = kFewCluster / 2;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(p.splits);
-  config.gridDim = dim3(static_cast<unsigned>(p.kv_heads * p.splits), static_cast<unsigned>(row_tiles));
+  const int row_tiles = (p.m * group + S::kRows - 1) / S::kRows;
+  bool one_wave;
+  p.splits = few_ctas(span, static_cast<int64_t>(p.kv_heads) * row_tiles, [&](int ctas) { return few_resident<KV, D, NT>(dev, ctas); }, &one_wave);
+  if (p.m >= 4 && aligned16(out) && !few_rows_win(span, p.splits, one_wave, D)) return kUnsupportedFeature;
+  cudaLaunchAttribute cluster;
+  const cudaLaunchConfig_t config =
+      few_config<KV, D, NT>(&cluster, p.splits, dim3(static_cast<unsigned>(p.kv_heads * p.splits), static_cast<unsigned>(row_tiles)), st);
   if (cudaLaunchKernelEx(&config, kernel, p, group, out, gate) != cudaSuccess) return kDeviceError;
   return check_launch();
 }
 
 template <int KV>
-int launch_few(const AttnParams& p, int group, float* out, const float* gate, cudaStream_t st) {
+int launch_few(const AttnParams& p, long span, int group, float* out, const float* gate, cudaStream_t st) {
   if (p.m * group <= 8)
-    return p.head_dim == 256 ? launch_few_nt<KV, 256, 1>(p, group, out, gate, st) : launch_few_nt<KV, 128, 1>(p, group, out, gate, st);
-  return p.head_dim == 256 ? launch_few_nt<KV, 256, 2>(p, group, out, gate, st) : launch_few_nt<KV, 128, 2>(p, group, out, gate, st);
+    return p.head_dim == 256 ? launch_few_nt<KV, 256, 1>(p, span, group, out, gate, st) : launch_few_nt<KV, 128, 1>(p, span, group, out, gate, st);
+  return p.head_dim == 256 ? launch_few_nt<KV, 256, 2>(p, span, group, out, gate, st) : launch_few_nt<KV, 128, 2>(p, span, group, out, gate, st);
 }
 
 bool overlap(const void* a, size_t an, const void* b, size_t bn) {
   const auto *x = static_cast<const unsigned char*>(a), *y = static_cast<const unsigned char*>(b);
   return x < y + bn && y < x + an;
 }
-bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // Whether the result may be written while other CTAs still read their queries and the cache.  In place over q is fine (a
 // CTA or cluster reads its own rows before it writes them); any other overlap stays with the chunk kernel, whose merge
@@ -1128,12 +1147,10 @@ int attention_few(int kvkind, AttnParams p, float* out, const float* gate, cudaS
   const long span = p.causal && p.window != 0 && p.window < p.n ? p.window : p.n;
   if (kvkind < kKvFp8 || !aligned16(p.q) || !aligned16(p.k) || !aligned16(p.v) || !writes_apart(kvkind, p, out, gate))
     return kUnsupportedFeature;
-  p.splits = 1;
-  while (p.splits < kFewCluster && p.splits * kFewKeysPerCta < span) p.splits *= 2;
   switch (kvkind) {
-    case kKvFp8: return launch_few<kKvFp8>(p, group, out, gate, st);
-    case kKvInt8: return launch_few<kKvInt8>(p, group, out, gate, st);
-    default: return launch_few<kKvInt4>(p, group, out, gate, st);
+    case kKvFp8: return launch_few<kKvFp8>(p, span, group, out, gate, st);
+    case kKvInt8: return launch_few<kKvInt8>(p, span, group, out, gate, st);
+    default: return launch_few<kKvInt4>(p, span, group, out, gate, st);
   }
 }
 
@@ -1141,12 +1158,11 @@ int attention_tile(int kvkind, AttnParams p, float* out, const float* gate, cuda
   const int group = p.heads / p.kv_heads;
   const long rows = static_cast<long>(p.m) * group;
   const long span = static_cast<long>(tile_span(p.m, p.n, p.q_base, p.window, p.causal != 0, group));
-  // Below a few rows a CTA's 128-row tile is mostly empty, and a short call is over before the tile's start has paid
-  // off: measured (FP8, chunk kernel -> here) 8 rows x 200 keys 18 -> 20 us, 16 x 300 22.8 -> 23.8, 8 x 1024 28.9 -> 22.8,
-  // 4 x 4096 45 -> 30, 16 x 4096 150 -> 36 (24 heads over 4 of 256); 2 rows x 4096 29 -> 29.
-  // 16-byte pieces of q, the cache and the output; the chunk kernel takes what is not aligned.
-  if (kvkind == kKvF32 || p.m < 4 || static_cast<double>(p.m) * span * p.kv_heads * p.head_dim < 8.0e6 || !aligned16(p.q) ||
-      !aligned16(p.k) || !aligned16(p.v) || !aligned16(out))
+  // 16-byte pieces of q, the cache and the output; the other kernels take what is not aligned.  Below four rows a row tile is
+  // mostly empty: 2 rows x 4096 fp16 keys 35.7 us, chunk kernel 28.2.
+  const double products = static_cast<double>(p.m) * span * p.heads * p.head_dim;
+  if (kvkind == kKvF32 || p.m < 4 || products < tile_least(kvkind == kKvF16, p.m) || !aligned16(p.q) || !aligned16(p.k) ||
+      !aligned16(p.v) || !aligned16(out))
     return kUnsupportedFeature;
   if (!writes_apart(kvkind, p, out, gate)) return kUnsupportedFeature;
   static const int sms = [] {

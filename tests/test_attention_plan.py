@@ -48,3 +48,40 @@ def test_widest_window_and_no_mask(plan):
     """A window beyond every position is no window, up to the largest the entry points take."""
     wide = ["tile_span(512, 4096, 3584, %d, true, %d)" % (w, g) for w in (2**31 - 1, 2**31 - 18, 4096) for g in (1, 6, 8)]
     assert plan(*wide, "tile_span(8, 500, 0, 3, false, 2)") == [4096] * len(wide) + [500]
+
+
+def cluster_plan(span, clusters, resident):
+    """(CTAs per cluster, one wave) by the rule."""
+    most = 1
+    while most < 16 and most * 16 < span:
+        most *= 2
+    sizes = [c for c in (16, 8, 4, 2, 1) if c <= most and clusters <= resident[c]]
+    return (sizes[0], 1) if sizes else (min(most, 8), 0)
+
+
+# clusters of 1, 2, 4, 8, 16 CTAs that run at a time: a whole B200, one that takes no clusters of sixteen, a small partition
+DEVICES = [{1: 148, 2: 74, 4: 36, 8: 14, 16: 7}, {1: 148, 2: 74, 4: 36, 8: 14, 16: 0}, {1: 14, 2: 7, 4: 3, 8: 1, 16: 0}]
+
+
+@pytest.mark.parametrize("resident", DEVICES)
+def test_clusters_of_few_rows(plan, resident):
+    """A size the device does not take is never chosen, nor a reason to refuse a call that smaller ones serve; one that is
+    not needed is not asked for."""
+    cases = [(s, c) for s in (1, 16, 17, 100, 129, 4096, 2**31 - 1) for c in (1, 4, 7, 8, 14, 15, 36, 37, 100, 148, 149, 60000)]
+    lookup = "[&](int c) { asked = c > asked ? c : asked; return c == 1 ? %d : c == 2 ? %d : c == 4 ? %d : c == 8 ? %d : %d; }" % tuple(
+        resident[c] for c in (1, 2, 4, 8, 16))
+    got = plan(*("[] { int asked = 0; bool w; const int c = few_ctas(%d, %d, %s, &w); return c + 100 * w + 1000 * asked; }()" % (s, c, lookup)
+                 for s, c in cases))
+    for (span, clusters), v in zip(cases, got):
+        want, wave = cluster_plan(span, clusters, resident)
+        assert v % 100 == want and v // 100 % 10 == wave, (span, clusters)
+        assert v // 1000 <= max(1, 2 * span / 16)
+        assert resident[want] > 0
+
+
+def test_kernel_for_a_batch(plan):
+    """All clusters at a time and 512 keys of 256 elements a CTA (256 with one or two CTAs a cluster); fp16 row tiles."""
+    wins = [("4096, 8, true, 256", 1), ("4097, 8, true, 256", 0), ("8192, 8, true, 128", 1), ("512, 2, true, 256", 1), ("513, 2, true, 256", 0),
+            ("16, 1, true, 256", 1), ("16, 1, false, 256", 0), ("2147483647, 16, true, 256", 0)]
+    assert plan(*("few_rows_win(%s)" % a for a, _ in wins)) == [v for _, v in wins]
+    assert plan("tile_least(false, 4)", "tile_least(true, 4)", "tile_least(true, 16)") == [12000000, 45000000, 22000000]
