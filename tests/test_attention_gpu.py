@@ -229,9 +229,10 @@ def test_written_cache_feeds_attention(backend, oracle):
 
 # (m, n, heads, kv_heads, head_dim, q_base, window): the fewest rows the tile takes, a second row tile of four rows, one
 # head per kv head on a first chunk, a window that starts inside tiles, query rows past the cache, eight heads per kv
-# head over many chunks
+# head over many chunks, five and seven heads per kv head (a row tile ends inside a query row), one chunk
 BATCHES = [(4, 2100, 24, 4, 256, 2096, 0), (22, 400, 24, 4, 256, 378, 0), (130, 130, 8, 8, 128, 0, 0), (101, 1500, 16, 2, 128, 1399, 300),
-           (57, 160, 24, 4, 256, 120, 0), (129, 700, 4, 4, 128, 500, 130), (16, 2049, 16, 2, 256, 2033, 0)]
+           (57, 160, 24, 4, 256, 120, 0), (129, 700, 4, 4, 128, 500, 130), (16, 2049, 16, 2, 256, 2033, 0), (40, 900, 15, 3, 128, 860, 70),
+           (39, 640, 14, 2, 256, 601, 0), (600, 64, 4, 2, 128, 0, 0)]
 
 
 @pytest.mark.parametrize("fmt", [1, 2, 3, 4])
@@ -248,15 +249,20 @@ def test_batches_on_the_tensor_pipe(backend, oracle, fmt, m, n, heads, kv_heads,
 
 # (m, n, heads, kv_heads, head_dim, q_base, window): one key, fewer keys than a warp's sixteen, a chunk that ends inside a
 # warp's keys, eight rows of the sixteen over two row tiles, a window whose first keys leave chunks empty for the last row,
-# 64 chunks, the last of them empty
+# sixteen chunks of unequal length, query rows past the cache, five heads per kv head; then the first rows of a long cache,
+# where most CTAs of a cluster (counted on all keys) have none and still take part in the merge, in both row widths; sixteen
+# CTAs of which the last has no key; batches in several clusters a kv head of eight, four and two CTAs
 FEW = [(1, 1, 24, 4, 256, 0, 0), (1, 13, 8, 8, 128, 12, 0), (1, 1000, 8, 1, 128, 900, 0), (3, 333, 16, 2, 256, 330, 0),
-       (3, 500, 6, 1, 128, 450, 70), (1, 4097, 24, 4, 256, 4096, 0), (2, 64, 12, 4, 256, 70, 0)]
+       (3, 500, 6, 1, 128, 450, 70), (1, 4097, 24, 4, 256, 4096, 0), (2, 64, 12, 4, 256, 70, 0), (2, 700, 10, 2, 128, 698, 0),
+       (1, 4096, 8, 2, 128, 0, 0), (1, 4096, 24, 4, 256, 20, 0), (3, 4096, 16, 2, 128, 5, 0), (2, 3000, 24, 4, 256, 0, 0),
+       (1, 129, 8, 2, 128, 128, 0), (9, 150, 24, 4, 256, 141, 0), (70, 90, 16, 4, 128, 20, 0), (200, 70, 16, 4, 128, 0, 33)]
 
 
 @pytest.mark.parametrize("fmt", [2, 3, 4])
 @pytest.mark.parametrize("m,n,heads,kv_heads,head_dim,q_base,window", FEW)
 def test_few_rows_on_the_tensor_pipe(backend, oracle, fmt, m, n, heads, kv_heads, head_dim, q_base, window):
-    """One to three query rows (two binary16 terms per query element and weight, exact cache elements): fp32 rounding."""
+    """A cluster per kv head and sixteen (row, head) pairs (two binary16 terms per query element and weight, exact cache
+    elements): fp32 rounding."""
     g = np.random.default_rng(80 + fmt + n)
     q = g.standard_normal((m, heads * head_dim)).astype(np.float32) * np.float32(10.0) ** g.integers(-3, 2, (m, 1)).astype(np.float32)
     k, v, ks, vs = make_cache(g, fmt, n, kv_heads * head_dim)
@@ -346,6 +352,83 @@ def test_value_scales_at_the_ends_of_their_range(backend, oracle, fmt, exponent,
     y = device_attention(backend, fmt, q, k, v, ks, vs * factor, m, n, heads, kv_heads, head_dim, q_base, 0, True)
     assert np.isfinite(y).all()
     assert near_each(y / factor, r, head_dim)
+
+
+@pytest.mark.parametrize("fmt,scale,value", [(2, "k", np.nan), (2, "v", np.inf), (3, "k", np.nan), (3, "v", -np.inf), (4, "v", np.nan)])
+@pytest.mark.parametrize("m,n", [(120, 300), (2, 200)])
+def test_nonfinite_scales_reach_only_the_rows_that_see_them(backend, oracle, fmt, scale, value, m, n):
+    """A key in the middle of the rows' positions has a scale that is not finite: the rows before it are untouched, the
+    others get the oracle's infinities and NaN."""
+    g = np.random.default_rng(120 + fmt + m)
+    heads, kv_heads, head_dim = 8, 2, 128
+    q = g.standard_normal((m, heads * head_dim)).astype(np.float32)
+    k, v, ks, vs = make_cache(g, fmt, n, kv_heads * head_dim)
+    (ks if scale == "k" else vs)[n - m // 2] = value
+    y = device_attention(backend, fmt, q, k, v, ks, vs, m, n, heads, kv_heads, head_dim, n - m, 0, True)
+    r = oracle.attention(fmt, q, k, v, m, n, heads, kv_heads, head_dim, n - m, 0, True, ks, vs).reshape(y.shape)
+    clean = m - m // 2
+    assert near_each(y[:clean], r[:clean], head_dim)
+    assert not np.isfinite(y[clean:]).any()
+    assert np.array_equal(np.isnan(y), np.isnan(r)) and np.array_equal(np.isposinf(y), np.isposinf(r))
+
+
+@pytest.mark.parametrize("fmt,bad", [(4, False), (4, True), (3, False), (1, False), (2, True)])
+@pytest.mark.parametrize("m,n,heads,kv_heads,head_dim", SHAPES)
+def test_sigmoid_gate_inside_attention(backend, oracle, fmt, bad, m, n, heads, kv_heads, head_dim):
+    """attention and the sigmoid_gate of its output, queued side by side, run as one operation: in the tile's own output,
+    in the merge of its chunks and in a cluster's merge, also where a value that is not finite is among the keys."""
+    g = np.random.default_rng(130 + fmt + m)
+    q, gate = (g.standard_normal((m, heads * head_dim)).astype(np.float32) for _ in range(2))
+    k, v, ks, vs = make_cache(g, fmt, n, kv_heads * head_dim)
+    if bad and fmt == 4:
+        v[n - 1, 3] = 0x7F
+    elif bad:
+        vs[n - 1] = np.nan
+    up, out = backend.upload, backend.AllocateBuffer(m * heads * head_dim * 4)
+    bufs, tail = [up(q), up(k), up(v)], [n - m if n >= m else 0, 0, 0]
+    if fmt >= 2:
+        bufs += [up(ks), up(vs)]
+    gb = up(gate)
+
+    def kernels(gated):
+        before = backend.LaunchStats()[1]
+        run(backend, "attention" if fmt < 2 else QUANT_ID[fmt], bufs + [out],
+            [m, n, heads, kv_heads, head_dim] + tail + ([fmt, 1] if fmt < 2 else [QUANT_KIND[fmt]]))
+        if gated:
+            run(backend, "sigmoid_gate", [out, gb, out], [m * heads * head_dim])
+        backend.Synchronize()
+        return backend.LaunchStats()[1] - before
+    backend.Synchronize()
+    backend.SetDeferred(2)
+    try:
+        alone, merged = kernels(False), kernels(True)
+    finally:
+        backend.SetDeferred(0)
+    assert merged == alone
+    y = backend.download(out, np.float32, q.size).reshape(m, -1)
+    r = oracle.attention(fmt, q, k, v, m, n, heads, kv_heads, head_dim, tail[0], 0, True, ks, vs).reshape(m, -1)
+    r = oracle.sigmoid_gate(r.reshape(-1), gate.reshape(-1)).reshape(m, -1)
+    assert np.array_equal(np.isnan(y), np.isnan(r)) and np.isnan(y).any() == bad
+    assert near(np.nan_to_num(y), np.nan_to_num(r))
+
+
+@pytest.mark.parametrize("fmt", [3, 4])
+@pytest.mark.parametrize("over", ["q", "v"])
+@pytest.mark.parametrize("m,n,heads,kv_heads,head_dim", SHAPES)
+def test_result_over_an_input(backend, oracle, fmt, over, m, n, heads, kv_heads, head_dim):
+    """In place over the queries (a CTA or a cluster reads its own rows first), and over the values (everything is read
+    before anything is written)."""
+    g = np.random.default_rng(140 + fmt + m)
+    q = g.standard_normal((m, heads * head_dim)).astype(np.float32)
+    k, v, ks, vs = make_cache(g, fmt, n, kv_heads * head_dim)
+    q_base = n - m if n >= m else 0
+    qb, kb = backend.upload(q), backend.upload(k)
+    vb = backend.upload(np.concatenate([v.reshape(-1), np.zeros(max(16, q.nbytes - v.nbytes), np.uint8)]))
+    out = qb if over == "q" else vb
+    run(backend, QUANT_ID[fmt], [qb, kb, vb, backend.upload(ks), backend.upload(vs), out],
+        [m, n, heads, kv_heads, head_dim, q_base, 0, 0, QUANT_KIND[fmt]])
+    y = backend.download(out, np.float32, q.size).reshape(m, -1)
+    assert near(y, oracle.attention(fmt, q, k, v, m, n, heads, kv_heads, head_dim, q_base, 0, True, ks, vs).reshape(m, -1))
 
 
 def decoded64(fmt, cache, scale, n):
