@@ -87,7 +87,7 @@ def test_golden_cases_every_format(backend):
 
 @pytest.mark.parametrize("fmt", [0, 1, 2, 3, 4])
 def test_decode_row_over_a_long_cache(backend, oracle, fmt):
-    """One query row, 24 heads over 4 kv heads of 256, 4096 keys: the key range is cut into 32 chunks."""
+    """One query row, 24 heads over 4 kv heads of 256, 4096 keys: 64 chunks (fp32, fp16), a cluster of sixteen CTAs (the others)."""
     g = np.random.default_rng(10 + fmt)
     n, heads, kv_heads, head_dim = 4096, 24, 4, 256
     q = g.standard_normal((1, heads * head_dim)).astype(np.float32)
