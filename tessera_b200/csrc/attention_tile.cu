@@ -23,7 +23,8 @@
 // Not built: the same on tcgen05, whose A operand can lie in tensor memory (weights without shared memory) and whose per-tile
 // sums would be added to fp32 registers as here.  Open there: the leading terms of a score keep their accuracy for one MMA of 16
 // elements, so every such product would be read back from tensor memory by itself.
-// Bound: the tensor pipe, at the mma.sync rate: four MMAs where a plain product needs two (fp16: six).  512 rows over 4096
+// Bound: the tensor pipe as two warps a scheduler reach it with mma.sync (48 % busy, the rest fixed latencies and waits for the
+// pipe): four MMAs where a plain product needs two (fp16: six).  512 rows over 4096
 // keys, 24 heads of 256: FP8 423 us against the chunk kernel's 4470 (114 TFLOP/s of the contract's 48 GFLOP, 228 of the MMAs'),
 // fp16 589 us against 4615.  255 registers a thread, 16 to 84 bytes of them spilled.
 #include <cuda_fp16.h>
