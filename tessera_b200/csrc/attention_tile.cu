@@ -26,7 +26,7 @@
 // Bound: the tensor pipe as two warps a scheduler reach it with mma.sync (48 % busy, the rest fixed latencies and waits for the
 // pipe): four MMAs where a plain product needs two (fp16: six).  512 rows over 4096
 // keys, 24 heads of 256: FP8 423 us against the chunk kernel's 4470 (114 TFLOP/s of the contract's 48 GFLOP, 228 of the MMAs'),
-// fp16 589 us against 4615.  255 registers a thread, 16 to 84 bytes of them spilled.
+// fp16 589 us against 4615.  255 registers a thread, 16 to 60 bytes spilled.
 #include <cuda_fp16.h>
 
 #include <atomic>
@@ -657,7 +657,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) attention_tile_kernel(const A
 // along g and are turned by movmatrix.  Two terms per query element and weight and exact cache elements as above; the MMAs
 // of four steps are added pairwise and the cluster's chunks without roundings.  One row of 24 heads over 4 of 256 and 4096 FP8
 // keys 11.7 us (chunk kernel 15.2) at 2.2e-7 against 64 bits (2.9e-7).  Bound: latency (64 CTAs, two trips a warp) and the
-// registers: 179 to 255 a thread, and with sixteen rows of 256 up to 432 bytes spilled.
+// registers: 179 to 255 a thread, and with sixteen rows of 256 up to 436 bytes spilled.
 constexpr int kFewWarps = 8, kFewKeys = 16;  // a warp's keys at a time
 
 template <int KV, int D, int NT>
